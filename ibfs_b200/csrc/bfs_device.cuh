@@ -38,7 +38,8 @@ constexpr int kDirBU = 1;
 constexpr int kMaxWords = 8;   // W = 256
 constexpr int kMaxPlanes = 16; // two-byte depths
 
-// Per-level counters, double-buffered by level parity.
+// Per-level counters, one of three sets per level (par_at): while level L runs,
+// L-1's set is still read and L+1's is being zeroed.
 struct Par {
   unsigned long long changed;  // vertices whose status changed
   unsigned long long mf;       // sum of their degrees (frontier edges)
@@ -48,7 +49,7 @@ struct Par {
   int32_t range_err;           // a level did not fit the depth type
   int32_t hq_cnt;              // deferred bottom-up hub chunks of this level
   int32_t pq_cnt;              // queued sparse-source push chunks of this level
-  int32_t pad;
+  int32_t t_cnt;               // vertices in the touched list of this level
   uint32_t scnt[kMaxWords * 32];  // per source: vertices it reached at the
                                   // previous level (sparse_count_phase)
 };
@@ -73,6 +74,8 @@ struct LoopState {
                               // (batch_end clears its unreachable sources' words)
   int32_t sparse_try;         // this bottom-up level follows a top-down one: count
                               // the sources' frontiers and pick the sparse ones
+  int32_t thin;               // `level` collects its changed vertices in the touched list
+  int32_t have_q;             // the queues of `level` were built by the previous inspect
   unsigned long long m_u, teps, prev_changed;
   unsigned long long t_lvl, t_mid;  // %globaltimer at the level start / inspect start
 };
@@ -83,11 +86,13 @@ struct __align__(256) Ctl {
   unsigned int bar_gen;
   int err;
   int pad0;
-  Par par[2];
+  Par par[3];
   int32_t qc[2][4];  // [consumer level parity][small, medium, large-chunks]
   unsigned long long pad1[4];
   LoopState ls;
 };
+
+__host__ __device__ inline Par* par_at(Ctl* ctl, int level) { return &ctl->par[level % 3]; }
 
 struct BatchRec {
   int32_t levels;     // levels expanded (incl. the last empty one)
@@ -109,8 +114,9 @@ struct GroupBufs {
   uint32_t* curr;    // [Vpad][WORDS]
   uint32_t* chg;     // 2 bitmaps of chg_stride words (level parity)
   uint32_t* planes;  // depth bit-planes, plane b at b*plane_stride words
-  int32_t* qs;
-  int32_t* qm;
+  int32_t* q;        // [V] frontier queue: small vertices from the front, medium
+                     // ones from the back (a vertex is in one class only)
+  int32_t* tl;       // [V] touched list of a thin top-down level
   int2* ql;
   int2* hq;          // deferred bottom-up hub chunks (v, chunk)
   Ctl* ctl;
@@ -378,32 +384,58 @@ static __device__ __noinline__ bool team_barrier(Ctl* ctl, unsigned nblocks,
   return s_ok != 0;
 }
 
-// CTA-wide sum of a 64-bit value, then one atomicAdd by thread 0.
-__device__ __forceinline__ void cta_add_u64(unsigned long long* dst, unsigned long long x) {
-  __shared__ unsigned long long s_red[32];
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+// A level's counters, summed over the CTA and added to `par` (every thread
+// calls it).  A CTA that changed nothing -- most of them on a thin level --
+// leaves after one barrier; otherwise the warps' sums meet in shared memory
+// behind a second one and one thread per counter issues its atomic.
+template <int WORDS>
+__device__ __forceinline__ void cta_flush(Par* par, unsigned long long cnt, unsigned long long mf,
+                                          unsigned long long cdeg, unsigned long long teps,
+                                          const uint32_t (&fm)[WORDS]) {
+  __shared__ unsigned long long s_c[32][4];
+  __shared__ uint32_t s_f[32][WORDS];
+  bool any = cnt != 0;
+#pragma unroll
+  for (int k = 0; k < WORDS; k++) any |= fm[k] != 0u;
+  if (!__syncthreads_or(any)) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) s_red[w] = x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long t = 0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += s_red[i];
-    if (t) atomicAdd(dst, t);
+  if (__any_sync(0xFFFFFFFFu, any)) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
+      mf += __shfl_xor_sync(0xFFFFFFFFu, mf, o);
+      cdeg += __shfl_xor_sync(0xFFFFFFFFu, cdeg, o);
+      teps += __shfl_xor_sync(0xFFFFFFFFu, teps, o);
+    }
+    if (l == 0) {
+      s_c[w][0] = cnt;
+      s_c[w][1] = mf;
+      s_c[w][2] = cdeg;
+      s_c[w][3] = teps;
+    }
+#pragma unroll
+    for (int k = 0; k < WORDS; k++) {
+      const uint32_t r = __reduce_or_sync(0xFFFFFFFFu, fm[k]);
+      if (l == 0) s_f[w][k] = r;
+    }
+  } else {
+    if (l < 4) s_c[w][l] = 0;
+    if (l < WORDS) s_f[w][l] = 0;
   }
-}
-
-__device__ __forceinline__ void cta_or_u32(uint32_t* dst, uint32_t x) {
-  __shared__ uint32_t s_or[32];
-  x = __reduce_or_sync(0xFFFFFFFFu, x);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   __syncthreads();
-  if (l == 0) s_or[w] = x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  const int nw = blockDim.x >> 5;
+  if (threadIdx.x < 4) {
+    unsigned long long t = 0;
+    for (int i = 0; i < nw; i++) t += s_c[i][threadIdx.x];
+    unsigned long long* dst = threadIdx.x == 0   ? &par->changed
+                              : threadIdx.x == 1 ? &par->mf
+                              : threadIdx.x == 2 ? &par->cdeg
+                                                 : &par->teps;
+    if (t) atomicAdd(dst, t);
+  } else if (threadIdx.x >= 32 && threadIdx.x < 32 + WORDS) {
     uint32_t t = 0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) t |= s_or[i];
-    if (t) atomicOr(dst, t);
+    for (int i = 0; i < nw; i++) t |= s_f[i][threadIdx.x - 32];
+    if (t) atomicOr(&par->fmask[threadIdx.x - 32], t);
   }
 }
 
@@ -455,16 +487,19 @@ __host__ __device__ inline int choose_dir(int next_level, int prev_dir,
 }
 
 // ---------------------------------------------------------------------------
-// Phase: seed the sources of one batch (curr bits + level-0 changed bits).
+// Phase: seed the sources of one batch (curr bits + level-0 changed bits, and
+// the touched list when the schedule inspects level 0 from it).
 // ---------------------------------------------------------------------------
-template <int WORDS>
+template <int WORDS, bool THIN>
 __device__ void seed_phase(const Params& p, const GroupBufs& gb,
                            const int32_t* src_b, int n_b, const Team& t) {
   uint32_t* chg0 = chg_at(gb, p, 0);
   for (long long i = t.tid; i < n_b; i += t.nthreads) {
     const int32_t v = src_b[i];
     atomicOr(gb.curr + (size_t)v * WORDS + (i >> 5), 1u << (i & 31));
-    atomicOr(chg0 + (v >> 5), 1u << (v & 31));
+    const uint32_t bit = 1u << (v & 31);
+    const uint32_t old = atomicOr(chg0 + (v >> 5), bit);
+    if (THIN && !(old & bit)) gb.tl[atomicAdd(&gb.ctl->par[0].t_cnt, 1)] = v;
   }
 }
 
@@ -477,20 +512,16 @@ __device__ __forceinline__ void zero_plane_if_first(const Params& p, const Group
   }
 }
 
-// ---------------------------------------------------------------------------
-// Phase: inspect level L (reads the level-L bitmap, fixes last, updates the
-// depth bit-planes, counters).
-// ---------------------------------------------------------------------------
-// Per changed vertex v of level L: new bits, last = curr, counters, planes.
+// Inspect work of one changed vertex v of level L: new bits, last = curr,
+// counters, planes; deg = its degree.
 template <int WORDS>
 __device__ __forceinline__ void inspect_vertex(const Params& p, const GroupBufs& gb, long long v,
                                                int level, bool depth_ok,
                                                const uint32_t (&full)[WORDS], uint32_t (&fm)[WORDS],
                                                unsigned long long& mf, unsigned long long& cnt,
                                                unsigned long long& cdeg,
-                                               unsigned long long& teps,
-                                               uint32_t (&nb)[WORDS]) {
-  uint32_t c[WORDS], l[WORDS];
+                                               unsigned long long& teps, long long& deg) {
+  uint32_t c[WORDS], l[WORDS], nb[WORDS];
   ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
   ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
   bool comp = true;
@@ -503,7 +534,7 @@ __device__ __forceinline__ void inspect_vertex(const Params& p, const GroupBufs&
     fm[k] |= nb[k];
   }
   st_status<WORDS>(gb.last + (size_t)v * WORDS, c);
-  const long long deg = p.beg[v + 1] - p.beg[v];
+  deg = p.beg[v + 1] - p.beg[v];
   mf += deg;
   cnt += 1;
   teps += (unsigned long long)deg * pop;
@@ -538,74 +569,44 @@ __device__ __forceinline__ void inspect_vertex(const Params& p, const GroupBufs&
 }
 
 // ---------------------------------------------------------------------------
-// Phase: inspect level L (reads the level-L bitmap, fixes last, updates the
-// depth bit-planes, counters).  Every warp step takes 32 bitmap words (1024
-// vertices) and compacts their set bits across the warp: lane j of round k
-// inspects the (32k + j)-th changed vertex of the chunk, found by a binary
-// search over the warp's inclusive bit counts (per-lane shuffles) and
-// __fns within the owning word.  All 32 lanes work on a changed vertex in
-// every full round whatever the density or the spread of the changed set,
-// so a frontier scattered thinly over the whole graph (a grid late in a
-// traversal, a power-law graph's tail) costs rounds of 32 vertices, not
-// one mostly idle round per non-empty word.
-//
-// LEAN selects the walk of the persistent kernel instead, whose budget of
-// 64 registers per thread (2 x 512 threads per SM) has no room for the
-// compaction: lanes map to the bits of one word, one word per warp step
-// (`dense`, many changed vertices) or the non-empty words of 128-word
-// blocks (few changed vertices).
+// Changed-vertex bitmap walk.  A warp takes `wpc` bitmap words per step and
+// writes the ids of their set bits, compacted, into its own piece of shared
+// memory, so that all lanes have a changed vertex in every full round of 32,
+// however thinly the set is spread.  wpc is kWalkWords on large graphs; on
+// small ones it
+// shrinks until every warp of the team has a step, because a step's rounds
+// are serial.  body(first vertex, ids, count) runs once per step.  A step is
+// 8 words: the lists of 16 warps then take 8 KB, so that the walks leave L1 to
+// the bottom-up kernels that share the SM with them (four groups of R-MAT
+// scale 24: 29.9 / 29.6 / 29.4 ms per run with steps of 32 / 16 / 8 words).
 // ---------------------------------------------------------------------------
-template <int WORDS, bool LEAN>
-__device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, int n_b,
-                              int level, bool depth_ok, bool dense, const Team& t) {
-  uint32_t full[WORDS];
-#pragma unroll
-  for (int k = 0; k < WORDS; k++) full[k] = full_word(n_b, k);
-  unsigned long long mf = 0, cnt = 0, cdeg = 0, teps = 0;
-  uint32_t fm[WORDS];
-#pragma unroll
-  for (int k = 0; k < WORDS; k++) fm[k] = 0;
-  const uint32_t* chg = chg_at(gb, p, level);
-  // the bitmap of level+1 (last used by level-1's expand) must start empty:
-  // bottom-up merges into it with atomics
-  zero_words(chg_at(gb, p, level + 1), p.chg_stride, t);
+constexpr int kWalkWords = 8;                     // bitmap words of one step at most
+constexpr int kWalkIds = kWalkWords * 32;         // ids of one step at most
+constexpr int kWalkWarps = 16;                    // warps per CTA at most (512 threads)
+
+__device__ __forceinline__ int walk_words(long long nchg, long long nwarps) {
+  int w = kWalkWords;
+  while (w > 1 && nchg < (long long)w * nwarps) w >>= 1;
+  return w;
+}
+
+// One warp's piece of the id lists (a function of its own, so that every walk
+// of a kernel shares one array).
+__device__ __forceinline__ uint16_t* walk_ids() {
+  __shared__ uint16_t s_ids[kWalkWarps][kWalkIds];
+  return s_ids[threadIdx.x >> 5];
+}
+
+template <class Body>
+__device__ __forceinline__ void walk_changed(const uint32_t* chg, long long nchg, const Team& t,
+                                             Body&& body) {
+  uint16_t* ids = walk_ids();
   const int lane = t.lane;
-  uint32_t nbx[WORDS];  // the new bits of the vertex a lane inspected (unused here)
-  if (LEAN && dense) {
-    for (long long w = t.warp; w < p.nchg; w += t.nwarps) {
-      const uint32_t bits = __ldcg(chg + w);
-      if (!bits) continue;
-      const long long v = w * 32 + lane;
-      if ((bits >> lane) & 1u)
-        inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, nbx);
-    }
-  } else if (LEAN) {
-    const long long nblk = (p.nchg + 127) / 128;
-    for (long long blk = t.warp; blk < nblk; blk += t.nwarps) {
-      const uint4 q4 = __ldcg(reinterpret_cast<const uint4*>(chg) + blk * 32 + lane);
-      uint32_t nzl = __ballot_sync(0xFFFFFFFFu, (q4.x | q4.y | q4.z | q4.w) != 0u);
-      while (nzl) {
-        const int src = __ffs(nzl) - 1;
-        nzl &= nzl - 1;
-        const uint32_t b0 = __shfl_sync(0xFFFFFFFFu, q4.x, src);
-        const uint32_t b1 = __shfl_sync(0xFFFFFFFFu, q4.y, src);
-        const uint32_t b2 = __shfl_sync(0xFFFFFFFFu, q4.z, src);
-        const uint32_t b3 = __shfl_sync(0xFFFFFFFFu, q4.w, src);
-        const long long w0 = blk * 128 + src * 4;
-        if ((b0 >> lane) & 1u)
-          inspect_vertex<WORDS>(p, gb, (w0 + 0) * 32 + lane, level, depth_ok, full, fm, mf, cnt, cdeg, teps, nbx);
-        if ((b1 >> lane) & 1u)
-          inspect_vertex<WORDS>(p, gb, (w0 + 1) * 32 + lane, level, depth_ok, full, fm, mf, cnt, cdeg, teps, nbx);
-        if ((b2 >> lane) & 1u)
-          inspect_vertex<WORDS>(p, gb, (w0 + 2) * 32 + lane, level, depth_ok, full, fm, mf, cnt, cdeg, teps, nbx);
-        if ((b3 >> lane) & 1u)
-          inspect_vertex<WORDS>(p, gb, (w0 + 3) * 32 + lane, level, depth_ok, full, fm, mf, cnt, cdeg, teps, nbx);
-      }
-    }
-  } else {
-  const long long nchunk = (p.nchg + 31) / 32;  // whole chunks lie inside chg_stride
-  for (long long c = t.warp; c < nchunk; c += t.nwarps) {
-    const uint32_t word = __ldcg(chg + c * 32 + lane);
+  const int wpc = walk_words(nchg, t.nwarps);
+  const long long nstep = (nchg + wpc - 1) / wpc;
+  for (long long c = t.warp; c < nstep; c += t.nwarps) {
+    const long long w = c * wpc + lane;
+    uint32_t word = (lane < wpc && w < nchg) ? __ldcg(chg + w) : 0u;
     if (__ballot_sync(0xFFFFFFFFu, word != 0u) == 0u) continue;
     const int own = __popc(word);
     int incl = own;
@@ -614,48 +615,124 @@ __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, in
       const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
       if (lane >= o) incl += y;
     }
-    const int excl = incl - own;
     const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    for (int base = 0; base < total; base += 32) {
-      const int r = base + lane;
-      // owner = number of lanes whose inclusive count is <= r
-      int lo = 0;
-#pragma unroll
-      for (int step = 16; step >= 1; step >>= 1) {
-        const int probe = __shfl_sync(0xFFFFFFFFu, incl, lo + step - 1);
-        if (probe <= r) lo += step;
-      }
-      const uint32_t w = __shfl_sync(0xFFFFFFFFu, word, lo);
-      const int e = __shfl_sync(0xFFFFFFFFu, excl, lo);
-      if (r < total) {
-        const int bit = (int)__fns(w, 0u, r - e + 1);
-        const long long v = (c * 32 + lo) * 32 + bit;
-        inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, nbx);
-      }
+    int at = incl - own;
+    while (word) {
+      ids[at++] = (uint16_t)(lane * 32 + __ffs(word) - 1);
+      word &= word - 1;
     }
+    __syncwarp();
+    body(c * wpc * 32, ids, total);
+    __syncwarp();  // the next step overwrites ids
   }
-  }
-  if (!depth_ok && cnt) par->range_err = 1;
-  cta_add_u64(&par->changed, cnt);
-  cta_add_u64(&par->mf, mf);
-  cta_add_u64(&par->cdeg, cdeg);
-  cta_add_u64(&par->teps, teps);
-#pragma unroll
-  for (int k = 0; k < WORDS; k++) cta_or_u32(&par->fmask[k], fm[k]);
 }
 
-// Whether the lean inspect of the next level should use the dense walk: its
-// changed set is at most the previous frontier's neighbourhood.
-__host__ __device__ inline bool inspect_dense(unsigned long long prev_mf, long long V) {
-  return prev_mf * 16ull > (unsigned long long)V;
+// Degree class of a frontier vertex (td_inspect, inspector.cuh:534-626):
+// deg < sml -> small (0), deg > lrg -> large (2), else medium (1); vertices
+// without edges are dropped (-1).
+__device__ __forceinline__ int deg_class(const Params& p, long long deg) {
+  return deg <= 0 ? -1 : deg < p.sml ? 0 : deg <= p.lrg ? 1 : 2;
+}
+
+// Append one vertex per lane (cls -1: none) to the queues: ballots, and one
+// atomic per class, the three of them issued together by three lanes.
+__device__ __forceinline__ void q_append(const Params& p, const GroupBufs& gb, int32_t* qc,
+                                         int lane, int32_t v, long long deg, int cls) {
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, cls == 0);
+  const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, cls == 1);
+  const uint32_t m2 = __ballot_sync(0xFFFFFFFFu, cls == 2);
+  if (!(m0 | m1 | m2)) return;
+  int nch = 0, incl = 0, total = 0;
+  if (m2) {  // large vertices are cut into chunks of p.chunk edges
+    nch = cls == 2 ? (int)((deg + p.chunk - 1) / p.chunk) : 0;
+    incl = nch;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+  }
+  const int add = lane == 0 ? __popc(m0) : lane == 1 ? __popc(m1) : lane == 2 ? total : 0;
+  int base = 0;
+  if (add) base = atomicAdd(&qc[lane], add);
+  const int b0 = __shfl_sync(0xFFFFFFFFu, base, 0);
+  const int b1 = __shfl_sync(0xFFFFFFFFu, base, 1);
+  const int b2 = __shfl_sync(0xFFFFFFFFu, base, 2);
+  if (cls == 0) gb.q[b0 + __popc(m0 & lt)] = v;
+  else if (cls == 1) gb.q[p.V - 1 - (b1 + __popc(m1 & lt))] = v;
+  else if (cls == 2)
+    for (int c = 0; c < nch; c++) gb.ql[b2 + incl - nch + c] = make_int2(v, c);
 }
 
 // ---------------------------------------------------------------------------
-// Phase: build the joint frontier queues for top-down level L from the
-// level-(L-1) bitmap (warp-ballot compaction, degree classes as td_inspect,
-// inspector.cuh:534-626: deg < sml -> small, deg > lrg -> large, else
-// medium, deg 0 dropped).  Large vertices are cut into chunks of p.chunk
-// edges.  Clears the level-L bitmap that the top-down pass will fill.
+// Phase: inspect level L.  Fixes last, updates the depth bit-planes and the
+// counters of every changed vertex.
+//   thin levels (kThinEdges) read the level's touched list and queue the
+//     vertices for the next top-down level on the way, so such a level reads
+//     nothing in proportion to the graph and needs no queue build;
+//   the others walk the level's bitmap.
+// What bounds a thin level is its chain of dependent L2 reads (queue entry,
+// offsets, column id, status, then list entry, statuses, planes), so the
+// step is one vertex per lane and 8 lanes per pushed small vertex.  A
+// 256 x 1024 grid without shortcuts (64 sources, 1269 levels, about 12,500
+// vertices each) went from 144 to 34 ms when its levels stopped walking the
+// whole bitmap with a few warps.
+// ---------------------------------------------------------------------------
+template <int WORDS>
+__device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, int n_b,
+                              int level, bool depth_ok, bool thin, int32_t* qc_next,
+                              const Team& t) {
+  uint32_t full[WORDS];
+#pragma unroll
+  for (int k = 0; k < WORDS; k++) full[k] = full_word(n_b, k);
+  unsigned long long mf = 0, cnt = 0, cdeg = 0, teps = 0;
+  uint32_t fm[WORDS];
+#pragma unroll
+  for (int k = 0; k < WORDS; k++) fm[k] = 0;
+  // the bitmap of level+1 (last used by level-1's expand) must start empty:
+  // bottom-up merges into it with atomics
+  zero_words(chg_at(gb, p, level + 1), p.chg_stride, t);
+  const int lane = t.lane;
+  if (thin) {
+    const int n = __ldcg(&par->t_cnt);
+    for (long long base = t.warp * 32; base < n; base += t.nwarps * 32) {
+      int32_t v = -1;
+      long long deg = 0;
+      if (base + lane < n) {
+        v = __ldcg(gb.tl + base + lane);
+        inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg);
+      }
+      q_append(p, gb, qc_next, lane, v, deg, deg_class(p, deg));
+    }
+  } else {
+    walk_changed(chg_at(gb, p, level), p.nchg, t,
+                 [&](long long v0, const uint16_t* ids, int total) {
+                   for (int r = lane; r < total; r += 32) {
+                     long long deg;
+                     inspect_vertex<WORDS>(p, gb, v0 + ids[r], level, depth_ok, full, fm, mf, cnt,
+                                           cdeg, teps, deg);
+                   }
+                 });
+  }
+  if (!depth_ok && cnt) par->range_err = 1;
+  cta_flush<WORDS>(par, cnt, mf, cdeg, teps, fm);
+}
+
+// A top-down level is thin when the frontier it pushes has at most this many
+// edges: its changed vertices then go through the touched list (one returned
+// atomic per first touch, one list append per warp step).  Above it the
+// appends to one counter cost more than a walk of the bitmap.  Measured with
+// the limit at 2^17 / 2^20 / 2^23 edges: R-MAT scale 22, 512 sources 5.10 /
+// 5.06 / 5.14 ms; grid 4096^2, 256 sources 156.1 / 154.1 / 157.9 ms; R-MAT
+// scale 20, 60 sources in 32-bit words 1.55 / 1.56 / 1.61 ms.
+constexpr unsigned long long kThinEdges = 1ull << 20;
+
+// ---------------------------------------------------------------------------
+// Phase: build the joint frontier queues of top-down level L from the
+// level-(L-1) bitmap.  The classes of a step's vertices are counted first,
+// so that a step of up to 256 vertices costs one round of three atomics
+// instead of one per 32 vertices.
 // ---------------------------------------------------------------------------
 // With `sync` (a top-down level right after a fused bottom-up level, which
 // left the new statuses in `last` and the previous ones in `curr`) every
@@ -665,68 +742,63 @@ __device__ inline void qbuild_phase(const Params& p, const GroupBufs& gb, int le
                                     int32_t* qc, const Team& t, bool sync = false) {
   const int lane = t.lane;
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t* prev = chg_at(gb, p, level - 1);
-  uint32_t* next = chg_at(gb, p, level);
-  const long long nblk = (p.nchg + 127) / 128;
-  for (long long blk = t.warp; blk < nblk; blk += t.nwarps) {
-   const uint4 q4 = __ldcg(reinterpret_cast<const uint4*>(prev) + blk * 32 + lane);
-   __stcg(reinterpret_cast<uint4*>(next) + blk * 32 + lane, make_uint4(0, 0, 0, 0));
-   uint32_t nzl = __ballot_sync(0xFFFFFFFFu, (q4.x | q4.y | q4.z | q4.w) != 0u);
-   while (nzl) {
-    const int src_lane = __ffs(nzl) - 1;
-    nzl &= nzl - 1;
-    const uint32_t qw[4] = {__shfl_sync(0xFFFFFFFFu, q4.x, src_lane),
-                            __shfl_sync(0xFFFFFFFFu, q4.y, src_lane),
-                            __shfl_sync(0xFFFFFFFFu, q4.z, src_lane),
-                            __shfl_sync(0xFFFFFFFFu, q4.w, src_lane)};
-    for (int kk = 0; kk < 4; kk++) {
-    const uint32_t bits = qw[kk];
-    if (!bits) continue;
-    const long long w = blk * 128 + src_lane * 4 + kk;
-    const long long v = w * 32 + lane;
-    const bool mine = (bits >> lane) & 1u;
-    long long deg = 0;
-    if (mine) deg = p.beg[v + 1] - p.beg[v];
-    if (sync && mine) {
-      uint32_t x[WORDS];
-      ld_status<WORDS>(gb.last + (size_t)v * WORDS, x);
-      st_status<WORDS>(gb.curr + (size_t)v * WORDS, x);
-    }
-    const int cls = (!mine || deg == 0) ? -1 : deg < p.sml ? 0 : deg <= p.lrg ? 1 : 2;
-    const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, cls == 0);
-    if (m0) {
-      const int leader = __ffs(m0) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(&qc[0], __popc(m0));
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (cls == 0) gb.qs[base + __popc(m0 & lt)] = (int32_t)v;
-    }
-    const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, cls == 1);
-    if (m1) {
-      const int leader = __ffs(m1) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(&qc[1], __popc(m1));
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (cls == 1) gb.qm[base + __popc(m1 & lt)] = (int32_t)v;
-    }
-    const uint32_t m2 = __ballot_sync(0xFFFFFFFFu, cls == 2);
-    if (m2) {
-      int nch = cls == 2 ? (int)((deg + p.chunk - 1) / p.chunk) : 0;
-      int incl = nch;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
+  walk_changed(chg_at(gb, p, level - 1), p.nchg, t,
+               [&](long long v0, uint16_t* ids, int total) {
+    // count the classes; the class stays in the id's top bits
+    int n0 = 0, n1 = 0, n2 = 0;
+    for (int r0 = 0; r0 < total; r0 += 32) {
+      int cls = -1, nch = 0;
+      if (r0 + lane < total) {
+        const uint32_t id = ids[r0 + lane];
+        const long long v = v0 + id;
+        const long long deg = p.beg[v + 1] - p.beg[v];
+        if (sync) {
+          uint32_t x[WORDS];
+          ld_status<WORDS>(gb.last + (size_t)v * WORDS, x);
+          st_status<WORDS>(gb.curr + (size_t)v * WORDS, x);
+        }
+        cls = deg_class(p, deg);
+        if (cls == 2) nch = (int)((deg + p.chunk - 1) / p.chunk);
+        ids[r0 + lane] = (uint16_t)(id | (uint32_t)(cls + 1) << 10);
       }
-      const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-      int base = 0;
-      if (lane == 0) base = atomicAdd(&qc[2], total);
-      base = __shfl_sync(0xFFFFFFFFu, base, 0);
-      const int first = base + incl - nch;
-      for (int c = 0; c < nch; c++) gb.ql[first + c] = make_int2((int)v, c);
+      n0 += __popc(__ballot_sync(0xFFFFFFFFu, cls == 0));
+      n1 += __popc(__ballot_sync(0xFFFFFFFFu, cls == 1));
+      if (__any_sync(0xFFFFFFFFu, cls == 2)) n2 += __reduce_add_sync(0xFFFFFFFFu, nch);
     }
+    __syncwarp();
+    const int add = lane == 0 ? n0 : lane == 1 ? n1 : lane == 2 ? n2 : 0;
+    int base = 0;
+    if (add) base = atomicAdd(&qc[lane], add);
+    int b0 = __shfl_sync(0xFFFFFFFFu, base, 0);
+    int b1 = __shfl_sync(0xFFFFFFFFu, base, 1);
+    int b2 = __shfl_sync(0xFFFFFFFFu, base, 2);
+    for (int r0 = 0; r0 < total; r0 += 32) {
+      int cls = -1;
+      int32_t v = 0;
+      if (r0 + lane < total) {
+        const uint32_t id = ids[r0 + lane];
+        v = (int32_t)(v0 + (id & 1023u));
+        cls = (int)(id >> 10) - 1;
+      }
+      const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, cls == 0);
+      const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, cls == 1);
+      if (cls == 0) gb.q[b0 + __popc(m0 & lt)] = v;
+      if (cls == 1) gb.q[p.V - 1 - (b1 + __popc(m1 & lt))] = v;
+      b0 += __popc(m0);
+      b1 += __popc(m1);
+      if (__any_sync(0xFFFFFFFFu, cls == 2)) {
+        const int nch =
+            cls == 2 ? (int)((p.beg[v + 1] - p.beg[v] + p.chunk - 1) / p.chunk) : 0;
+        int incl = nch;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        for (int c = 0; c < nch; c++) gb.ql[b2 + incl - nch + c] = make_int2(v, c);
+        b2 += __shfl_sync(0xFFFFFFFFu, incl, 31);
+      }
     }
-   }
-  }
+  });
 }
 
 // Fire-and-forget ORs (red: no value comes back, so nothing waits on them).
@@ -747,11 +819,17 @@ __device__ __forceinline__ void red_or_u64(unsigned long long* p, unsigned long 
 // reductions whose old value is never needed: the thread issues them and
 // goes on instead of waiting for L2 round trips.  A stale s (fewer bits)
 // costs at most one redundant OR.
+//
+// THIN (the level keeps a touched list): the bitmap OR returns the old word,
+// which says whether this push was the first to change u at this level, and
+// the warp appends those vertices to the list with one atomic per step.  All
+// 32 lanes call it together (cnt 0: nothing to push).
 constexpr int kTdStep = 4;  // edges one thread has in flight
-template <int WORDS>
-__device__ __forceinline__ void td_push_n(const GroupBufs& gb, uint32_t* chg,
+template <int WORDS, bool THIN>
+__device__ __forceinline__ void td_push_n(const GroupBufs& gb, uint32_t* chg, int32_t* t_cnt,
                                           const int32_t (&u)[kTdStep], int cnt,
                                           const uint32_t (&P)[WORDS]) {
+  uint32_t first = 0;  // bit i: u[i] changed here first
   uint32_t s[kTdStep][WORDS];
 #pragma unroll
   for (int i = 0; i < kTdStep; i++) {
@@ -778,7 +856,29 @@ __device__ __forceinline__ void td_push_n(const GroupBufs& gb, uint32_t* chg,
         if (n0 | n1) red_or_u64(q + k, ((unsigned long long)P[2 * k + 1] << 32) | P[2 * k]);
       }
     }
-    red_or_u32(chg + (u[i] >> 5), 1u << (u[i] & 31));
+    const uint32_t bit = 1u << (u[i] & 31);
+    if constexpr (THIN) {
+      if (!(atomicOr(chg + (u[i] >> 5), bit) & bit)) first |= 1u << i;
+    } else {
+      red_or_u32(chg + (u[i] >> 5), bit);
+    }
+  }
+  if constexpr (THIN) {
+    if (!__any_sync(0xFFFFFFFFu, first != 0u)) return;
+    const int lane = threadIdx.x & 31;
+    const int own = __popc(first);
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    int base = 0;
+    if (lane == 31) base = atomicAdd(t_cnt, incl);
+    base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - own;
+#pragma unroll
+    for (int i = 0; i < kTdStep; i++)
+      if ((first >> i) & 1u) gb.tl[base++] = u[i];
   }
 }
 
@@ -858,10 +958,11 @@ __device__ __forceinline__ void td_chunk(const Params& p, const GroupBufs& gb, i
 // on R-MAT scale 24 the top-down levels are bound by the random status
 // gathers, not by the column reads, and staging measured ~1 % slower.
 // ---------------------------------------------------------------------------
-template <int WORDS, bool STAGE = false>
-__device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const int32_t* qc,
-                         const Team& t) {
+template <int WORDS, bool STAGE, bool THIN>
+__device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int level,
+                                       const int32_t* qc, const Team& t) {
   uint32_t* chg = chg_at(gb, p, level);
+  int32_t* t_cnt = &par_at(gb.ctl, level)->t_cnt;
   const int nS = __ldcg(qc + 0), nM = __ldcg(qc + 1), nL = __ldcg(qc + 2);
   if (STAGE && p.td_stage) {
     __shared__ __align__(128) int32_t s_col[2][kStageInts];
@@ -904,7 +1005,8 @@ __device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const 
       if (s_fail) break;  // uniform
       const int32_t* sc = s_col[i & 1] + (b0 - a0);
       const int n = (int)(b1 - b0);
-      for (int j = threadIdx.x; j < n; j += kTdStep * blockDim.x) {
+      for (int j0 = 0; j0 < n; j0 += kTdStep * blockDim.x) {
+        const int j = j0 + (int)threadIdx.x;
         int32_t u[kTdStep];
         int cnt = 0;
 #pragma unroll
@@ -913,7 +1015,7 @@ __device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const 
           u[q] = jq < n ? sc[jq] : 0;
           cnt += jq < n ? 1 : 0;
         }
-        td_push_n<WORDS>(gb, chg, u, cnt, P);
+        td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
       }
       __syncthreads();  // buffer i & 1 is read: the copy of chunk i + 2 may reuse it
     }
@@ -930,7 +1032,8 @@ __device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const 
       td_chunk(p, gb, c, &v, &b0, &b1, &a0, &a1);
       uint32_t P[WORDS];
       ld_status<WORDS>(gb.last + (size_t)v * WORDS, P);
-      for (long long e = b0 + threadIdx.x; e < b1; e += (long long)kTdStep * blockDim.x) {
+      for (long long e0 = b0; e0 < b1; e0 += (long long)kTdStep * blockDim.x) {
+        const long long e = e0 + threadIdx.x;
         int32_t u[kTdStep];
         int cnt = 0;
 #pragma unroll
@@ -939,16 +1042,17 @@ __device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const 
           u[i] = ei < b1 ? __ldg(p.col + ei) : 0;
           cnt += ei < b1 ? 1 : 0;
         }
-        td_push_n<WORDS>(gb, chg, u, cnt, P);
+        td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
       }
     }
   }
   for (long long i = t.warp; i < nM; i += t.nwarps) {
-    const int32_t v = gb.qm[i];
+    const int32_t v = __ldcg(gb.q + (p.V - 1 - i));
     uint32_t P[WORDS];
     ld_status<WORDS>(gb.last + (size_t)v * WORDS, P);
     const long long b1 = p.beg[v + 1];
-    for (long long e = p.beg[v] + t.lane; e < b1; e += 32 * kTdStep) {
+    for (long long e0 = p.beg[v]; e0 < b1; e0 += 32 * kTdStep) {
+      const long long e = e0 + t.lane;
       int32_t u[kTdStep];
       int cnt = 0;
 #pragma unroll
@@ -957,22 +1061,44 @@ __device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const 
         u[j] = ej < b1 ? __ldg(p.col + ej) : 0;
         cnt += ej < b1 ? 1 : 0;
       }
-      td_push_n<WORDS>(gb, chg, u, cnt, P);
+      td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
     }
   }
-  for (long long i = t.tid; i < nS; i += t.nthreads) {
-    const int32_t v = gb.qs[i];
+  // A thread per small vertex; a thin level, whose queue leaves most threads
+  // of the team without one, gives it 8 lanes instead, so that its list is
+  // one step (32 edges) and not a chain of them.
+  const int lg = (THIN && (long long)nS * 8 <= t.nthreads) ? 3 : 0;
+  for (long long i0 = t.warp << (5 - lg); i0 < nS; i0 += t.nwarps << (5 - lg)) {
+    const long long i = i0 + (t.lane >> lg);
     uint32_t P[WORDS];
-    ld_status<WORDS>(gb.last + (size_t)v * WORDS, P);
-    const long long b1 = p.beg[v + 1];
-    for (long long e = p.beg[v]; e < b1; e += kTdStep) {
+    long long e = 0, b1 = 0;
+    if (i < nS) {
+      const int32_t v = __ldcg(gb.q + i);
+      ld_status<WORDS>(gb.last + (size_t)v * WORDS, P);
+      b1 = p.beg[v + 1];
+      e = p.beg[v] + (long long)kTdStep * (t.lane & ((1 << lg) - 1));
+    } else {
+#pragma unroll
+      for (int k = 0; k < WORDS; k++) P[k] = 0u;
+    }
+    while (__any_sync(0xFFFFFFFFu, e < b1)) {
       int32_t u[kTdStep];
-      const int cnt = (int)min((long long)kTdStep, b1 - e);
+      const int cnt = (int)max(0LL, min((long long)kTdStep, b1 - e));
 #pragma unroll
       for (int j = 0; j < kTdStep; j++) u[j] = j < cnt ? __ldg(p.col + e + j) : 0;
-      td_push_n<WORDS>(gb, chg, u, cnt, P);
+      td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
+      e += (long long)kTdStep << lg;
     }
   }
+}
+
+// A template instance per kind: the thin one's lists and votes cost the
+// large levels registers otherwise.
+template <int WORDS, bool STAGE = false>
+__device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const int32_t* qc,
+                         bool thin, const Team& t) {
+  if (thin) td_run<WORDS, false, true>(p, gb, level, qc, t);
+  else td_run<WORDS, STAGE, false>(p, gb, level, qc, t);
 }
 
 // Second bottom-up stage: the hubs that were still missing frontier bits
@@ -1438,12 +1564,11 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   }
   if constexpr (FUSED) {
     if (range) par->range_err = 1;
-    cta_add_u64(&par->changed, f_cnt);
-    cta_add_u64(&par->mf, f_mf);
-    cta_add_u64(&par->cdeg, f_cdeg);
-    cta_add_u64(&par->teps, f_teps);
-    __syncthreads();
-    if (threadIdx.x < WORDS && s_fm[threadIdx.x]) atomicOr(&par->fmask[threadIdx.x], s_fm[threadIdx.x]);
+    uint32_t fmo[WORDS];  // every thread holds the CTA's OR (s_fm is complete
+    __syncthreads();      // behind the barrier)
+#pragma unroll
+    for (int k = 0; k < WORDS; k++) fmo[k] = s_fm[k];
+    cta_flush<WORDS>(par, f_cnt, f_mf, f_cdeg, f_teps, fmo);
   }
 }
 
@@ -1506,12 +1631,7 @@ __device__ void bu_hub_epilogue(const Params& p, const GroupBufs& gb, Par* par, 
       }
     }
   }
-  cta_add_u64(&par->changed, cnt);
-  cta_add_u64(&par->mf, mf);
-  cta_add_u64(&par->cdeg, cdeg);
-  cta_add_u64(&par->teps, teps);
-#pragma unroll
-  for (int k = 0; k < WORDS; k++) cta_or_u32(&par->fmask[k], fm[k]);
+  cta_flush<WORDS>(par, cnt, mf, cdeg, teps, fm);
 }
 
 // ---------------------------------------------------------------------------
@@ -1671,12 +1791,10 @@ __device__ __forceinline__ void push_edge(const Params& p, const GroupBufs& gb, 
 template <int WORDS>
 __device__ __forceinline__ void push_acc_flush(const PushAcc& acc, Par* par) {
   if (acc.range) par->range_err = 1;
-  cta_add_u64(&par->changed, acc.cnt);
-  cta_add_u64(&par->mf, acc.mf);
-  cta_add_u64(&par->cdeg, acc.cdeg);
-  cta_add_u64(&par->teps, acc.teps);
+  uint32_t fm[WORDS];
 #pragma unroll
-  for (int k = 0; k < WORDS; k++) cta_or_u32(&par->fmask[k], acc.fm[k]);
+  for (int k = 0; k < WORDS; k++) fm[k] = acc.fm[k];
+  cta_flush<WORDS>(par, acc.cnt, acc.mf, acc.cdeg, acc.teps, fm);
 }
 
 template <int WORDS>

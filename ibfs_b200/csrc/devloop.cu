@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(512) k_dl_batch_init(Params p, int g, CondH h_
   zero_words(gb.chg, 2 * p.chg_stride, t);
   if (t.tid == 0) {
     Ctl* ctl = gb.ctl;
-    memset(&ctl->par[0], 0, sizeof(Par) * 2);
+    memset(&ctl->par[0], 0, sizeof(ctl->par));
     memset(&ctl->qc[0][0], 0, sizeof(ctl->qc));
     LoopState& ls = ctl->ls;
     ls.level = 0;
@@ -212,6 +212,8 @@ __global__ void __launch_bounds__(512) k_dl_batch_init(Params p, int g, CondH h_
     ls.sync = 0;
     for (int k = 0; k < kMaxWords; k++) ls.smask[k] = 0u;
     ls.sparse_try = 0;
+    ls.thin = 1;  // level 0: the seeds are its touched list
+    ls.have_q = 0;
     ls.t_lvl = ls.t_mid = global_ns();
     cudaGraphSetConditional(h_level, 1u);
   }
@@ -221,7 +223,7 @@ template <int WORDS>
 __global__ void __launch_bounds__(512) k_dl_seed(Params p, int g, CondH, CondH) {
   const GroupBufs gb = dl_bufs(p, g);
   const int b = gb.ctl->ls.batch;
-  seed_phase<WORDS>(p, gb, p.src + (long long)b * p.C, dl_batch_size(p, gb.ctl->ls, b),
+  seed_phase<WORDS, true>(p, gb, p.src + (long long)b * p.C, dl_batch_size(p, gb.ctl->ls, b),
                     make_team(blockIdx.x, gridDim.x));
 }
 
@@ -231,8 +233,9 @@ __global__ void DL_INSPECT_BOUNDS k_dl_inspect(Params p, int g, CondH, CondH) {
   Ctl* ctl = gb.ctl;
   const int b = ctl->ls.batch, level = ctl->ls.level;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ls.t_mid = global_ns();
-  inspect_phase<WORDS, false>(p, gb, &ctl->par[level & 1], dl_batch_size(p, ctl->ls, b), level,
-                              level <= depth_limit(p.db), false, make_team(blockIdx.x, gridDim.x));
+  inspect_phase<WORDS>(p, gb, par_at(ctl, level), dl_batch_size(p, ctl->ls, b), level,
+                       level <= depth_limit(p.db), ctl->ls.thin != 0, ctl->qc[(level + 1) & 1],
+                       make_team(blockIdx.x, gridDim.x));
 }
 
 // Top of a level: read the counters of the level just inspected, stop or
@@ -247,7 +250,7 @@ __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
   // a fused bottom-up level left its statuses in the other buffer
   const bool was_bu = IBFS_DL_FUSED_BU && level > 0 && ls.dir == kDirBU;
   if (was_bu) ls.flip ^= 1;
-  const Par& pr = ctl->par[level & 1];
+  const Par& pr = *par_at(ctl, level);
   const unsigned long long changed = pr.changed, mf = pr.mf, cdeg = pr.cdeg;
   ls.teps += pr.teps;
   ls.m_u = ls.m_u > cdeg ? ls.m_u - cdeg : 0ull;
@@ -276,8 +279,11 @@ __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
   ls.t_lvl = t_now;
   ls.err = err;
   if (!stop) {
-    memset((void*)&ctl->par[(level + 1) & 1], 0, sizeof(Par));
+    memset((void*)par_at(ctl, level + 1), 0, sizeof(Par));
     ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
+    // a thin level left the next level's queues behind
+    ls.have_q = (nd == kDirTD && ls.thin && ls.dir == kDirTD) ? 1 : 0;
+    ls.thin = (nd == kDirTD && mf <= kThinEdges) ? 1 : 0;
     ls.sync = (was_bu && nd == kDirTD) ? 1 : 0;  // top-down needs curr == last again
     ls.dir = nd;
     ls.level = level + 1;
@@ -293,6 +299,7 @@ __global__ void __launch_bounds__(512) k_dl_qbuild(Params p, int g, CondH, CondH
   const int level = gb.ctl->ls.level;
   const Team t = make_team(blockIdx.x, gridDim.x);
   zero_plane_if_first(p, gb, level, t);
+  if (gb.ctl->ls.have_q) return;  // uniform
   qbuild_phase<WORDS>(p, gb, level, gb.ctl->qc[level & 1], t, gb.ctl->ls.sync != 0);
 }
 
@@ -300,8 +307,8 @@ template <int WORDS>
 __global__ void DL_TD_BOUNDS k_dl_td(Params p, int g, CondH, CondH) {
   const GroupBufs gb = dl_bufs(p, g);
   const int level = gb.ctl->ls.level;
-  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1],
-                                      make_team(blockIdx.x, gridDim.x));
+  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], gb.ctl->ls.thin != 0,
+                        make_team(blockIdx.x, gridDim.x));
 }
 
 template <int WORDS>
@@ -310,16 +317,16 @@ __global__ void DL_BU_BOUNDS k_dl_bu(Params p, int g, CondH, CondH) {
   const LoopState& ls = gb.ctl->ls;
   const int level = ls.level;
   const Team t = make_team(blockIdx.x, gridDim.x);
-  const bool filt = bu_filter_level(p.bu_filter, gb.ctl->par[(level - 1) & 1].changed, p.V);
+  const bool filt = bu_filter_level(p.bu_filter, par_at(gb.ctl, level - 1)->changed, p.V);
   if (IBFS_DL_FUSED_BU) {
-    bu_phase<WORDS, true, true, IBFS_BU_HUB_BYTES / (4 * WORDS)>(p, gb, level, gb.ctl->par[(level - 1) & 1].fmask,
-                          &gb.ctl->par[level & 1].hq_cnt, t, &gb.ctl->par[level & 1],
+    bu_phase<WORDS, true, true, IBFS_BU_HUB_BYTES / (4 * WORDS)>(p, gb, level, par_at(gb.ctl, level - 1)->fmask,
+                          &par_at(gb.ctl, level)->hq_cnt, t, par_at(gb.ctl, level),
                           dl_batch_size(p, ls, ls.batch), level <= depth_limit(p.db), filt,
                           ls.smask);
   } else {
     zero_plane_if_first(p, gb, level, t);
-    bu_phase<WORDS, false, true>(p, gb, level, gb.ctl->par[(level - 1) & 1].fmask,
-                                 &gb.ctl->par[level & 1].hq_cnt, t, nullptr, 0, true, filt);
+    bu_phase<WORDS, false, true>(p, gb, level, par_at(gb.ctl, level - 1)->fmask,
+                                 &par_at(gb.ctl, level)->hq_cnt, t, nullptr, 0, true, filt);
   }
 }
 
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(512) k_dl_bu_hubs(Params p, int g, CondH, Cond
   const int b = ctl->ls.batch, level = ctl->ls.level;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ls.t_mid = global_ns();
   const bool sparse = dl_sparse(ctl->ls, WORDS);
-  bu_hub_epilogue<WORDS>(p, gb, &ctl->par[level & 1], dl_batch_size(p, ctl->ls, b), level,
+  bu_hub_epilogue<WORDS>(p, gb, par_at(ctl, level), dl_batch_size(p, ctl->ls, b), level,
                          level <= depth_limit(p.db), make_team(blockIdx.x, gridDim.x), sparse);
 }
 
@@ -339,10 +346,10 @@ template <int WORDS>
 __global__ void __launch_bounds__(512) k_dl_bu_defer(Params p, int g, CondH, CondH) {
   const GroupBufs gb = dl_bufs(p, g);
   const int level = gb.ctl->ls.level;
-  if (gb.ctl->par[level & 1].hq_cnt == 0) return;  // uniform: nothing deferred
-  bu_defer_phase<WORDS, true>(p, gb, level, gb.ctl->par[(level - 1) & 1].fmask,
-                              &gb.ctl->par[level & 1].hq_cnt, make_team(blockIdx.x, gridDim.x),
-                              bu_filter_level(p.bu_filter, gb.ctl->par[(level - 1) & 1].changed,
+  if (par_at(gb.ctl, level)->hq_cnt == 0) return;  // uniform: nothing deferred
+  bu_defer_phase<WORDS, true>(p, gb, level, par_at(gb.ctl, level - 1)->fmask,
+                              &par_at(gb.ctl, level)->hq_cnt, make_team(blockIdx.x, gridDim.x),
+                              bu_filter_level(p.bu_filter, par_at(gb.ctl, level - 1)->changed,
                                               p.V),
                               gb.ctl->ls.smask);
 }
@@ -355,7 +362,7 @@ __global__ void __launch_bounds__(512) k_dl_sparse_count(Params p, int g, CondH,
   Ctl* ctl = gb.ctl;
   if (!ctl->ls.sparse_try) return;  // uniform
   const int level = ctl->ls.level;
-  sparse_count_phase<WORDS>(p, gb, &ctl->par[level & 1], level, make_team(blockIdx.x, gridDim.x));
+  sparse_count_phase<WORDS>(p, gb, par_at(ctl, level), level, make_team(blockIdx.x, gridDim.x));
 }
 
 __global__ void k_dl_sparse_decide(Params p, int g, CondH, CondH) {
@@ -363,7 +370,7 @@ __global__ void k_dl_sparse_decide(Params p, int g, CondH, CondH) {
   Ctl* ctl = p.groups[g].ctl;
   LoopState& ls = ctl->ls;
   if (!ls.sparse_try) return;
-  const Par& pr = ctl->par[ls.level & 1];
+  const Par& pr = *par_at(ctl, ls.level);
   const int nsrc = ls.nb;
   unsigned long long tot = 0;
   for (int i = 0; i < nsrc; i++) tot += pr.scnt[i];
@@ -395,7 +402,7 @@ __global__ void __launch_bounds__(512) k_dl_push_queue(Params p, int g, CondH, C
   const LoopState& ls = ctl->ls;
   if (!dl_sparse(ls, WORDS)) return;  // uniform
   const int level = ls.level;
-  push_queue_phase<WORDS>(p, gb, &ctl->par[level & 1], dl_batch_size(p, ls, ls.batch), level,
+  push_queue_phase<WORDS>(p, gb, par_at(ctl, level), dl_batch_size(p, ls, ls.batch), level,
                           level <= depth_limit(p.db), ls.smask,
                           make_team(blockIdx.x, gridDim.x));
 }
@@ -407,8 +414,8 @@ __global__ void __launch_bounds__(512) k_dl_push_run(Params p, int g, CondH, Con
   const LoopState& ls = ctl->ls;
   if (!dl_sparse(ls, WORDS)) return;  // uniform
   const int level = ls.level;
-  if (ctl->par[level & 1].pq_cnt == 0) return;  // uniform
-  push_run_phase<WORDS>(p, gb, &ctl->par[level & 1], dl_batch_size(p, ls, ls.batch), level,
+  if (par_at(ctl, level)->pq_cnt == 0) return;  // uniform
+  push_run_phase<WORDS>(p, gb, par_at(ctl, level), dl_batch_size(p, ls, ls.batch), level,
                         level <= depth_limit(p.db), ls.smask, make_team(blockIdx.x, gridDim.x));
 }
 

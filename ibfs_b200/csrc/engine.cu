@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(512) k_seed(Params p, int b) {
   const Team t = make_team(blockIdx.x, gridDim.x);
   const long long k0 = (long long)b * p.C;
   const int n_b = (int)min((long long)p.C, p.n_total - k0);
-  seed_phase<WORDS>(p, p.groups[0], p.src + k0, n_b, t);
+  seed_phase<WORDS, false>(p, p.groups[0], p.src + k0, n_b, t);
 }
 
 template <int WORDS>
@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(512) k_inspect(Params p, GroupBufs gb, int b, 
   const Team t = make_team(blockIdx.x, gridDim.x);
   const long long k0 = (long long)b * p.C;
   const int n_b = (int)min((long long)p.C, p.n_total - k0);
-  inspect_phase<WORDS, false>(p, gb, &gb.ctl->par[level & 1], n_b, level,
-                              level <= depth_limit(p.db), false, t);
+  inspect_phase<WORDS>(p, gb, par_at(gb.ctl, level), n_b, level, level <= depth_limit(p.db), false,
+                       nullptr, t);
 }
 
 __global__ void __launch_bounds__(512) k_qbuild(Params p, GroupBufs gb, int level) {
@@ -62,24 +62,24 @@ __global__ void __launch_bounds__(512) k_qbuild(Params p, GroupBufs gb, int leve
 template <int WORDS>
 __global__ void __launch_bounds__(512) k_td(Params p, GroupBufs gb, int level) {
   const Team t = make_team(blockIdx.x, gridDim.x);
-  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], t);
+  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], false, t);
 }
 
 template <int WORDS>
 __global__ void __launch_bounds__(512) k_bu(Params p, GroupBufs gb, int level) {
   const Team t = make_team(blockIdx.x, gridDim.x);
-  bu_phase<WORDS, false, true>(p, gb, level, gb.ctl->par[(level - 1) & 1].fmask,
-                               &gb.ctl->par[level & 1].hq_cnt, t, nullptr, 0, true,
-                               bu_filter_level(p.bu_filter, gb.ctl->par[(level - 1) & 1].changed,
+  bu_phase<WORDS, false, true>(p, gb, level, par_at(gb.ctl, level - 1)->fmask,
+                               &par_at(gb.ctl, level)->hq_cnt, t, nullptr, 0, true,
+                               bu_filter_level(p.bu_filter, par_at(gb.ctl, level - 1)->changed,
                                                p.V));
 }
 
 template <int WORDS>
 __global__ void __launch_bounds__(512) k_bu_defer(Params p, GroupBufs gb, int level) {
   const Team t = make_team(blockIdx.x, gridDim.x);
-  bu_defer_phase<WORDS, true>(p, gb, level, gb.ctl->par[(level - 1) & 1].fmask,
-                              &gb.ctl->par[level & 1].hq_cnt, t,
-                              bu_filter_level(p.bu_filter, gb.ctl->par[(level - 1) & 1].changed,
+  bu_defer_phase<WORDS, true>(p, gb, level, par_at(gb.ctl, level - 1)->fmask,
+                              &par_at(gb.ctl, level)->hq_cnt, t,
+                              bu_filter_level(p.bu_filter, par_at(gb.ctl, level - 1)->changed,
                                               p.V));
 }
 
@@ -167,10 +167,10 @@ struct PinBuf {
 };
 
 struct GroupMem {
-  DevBuf last, curr, chg, qs, qm, ql, hq, ctl, planes;
+  DevBuf last, curr, chg, q, tl, ql, hq, ctl, planes;
   void release() {
-    last.release(); curr.release(); chg.release(); qs.release();
-    qm.release(); ql.release(); hq.release(); ctl.release(); planes.release();
+    last.release(); curr.release(); chg.release(); q.release();
+    tl.release(); ql.release(); hq.release(); ctl.release(); planes.release();
   }
 };
 
@@ -334,8 +334,8 @@ static ibfs_status ensure_workspace(ibfs_graph* g, const RunPlan& rp, const ibfs
     if ((s = m.chg.ensure(2 * nchg * 4)) != IBFS_OK) return s;
     if ((s = m.planes.ensure((size_t)(rp.db == 1 ? 8 : 16) * vpad * rp.words * 4)) != IBFS_OK)
       return s;
-    if ((s = m.qs.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
-    if ((s = m.qm.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
+    if ((s = m.q.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
+    if ((s = m.tl.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
     if ((s = m.ql.ensure(capl * 8)) != IBFS_OK) return s;
     if ((s = m.hq.ensure((size_t)g->defer_cap * 8)) != IBFS_OK) return s;
     if ((s = m.ctl.ensure(sizeof(Ctl))) != IBFS_OK) return s;
@@ -1026,8 +1026,8 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     hgb[i].last = m.last.as<uint32_t>();
     hgb[i].curr = m.curr.as<uint32_t>();
     hgb[i].chg = m.chg.as<uint32_t>();
-    hgb[i].qs = m.qs.as<int32_t>();
-    hgb[i].qm = m.qm.as<int32_t>();
+    hgb[i].q = m.q.as<int32_t>();
+    hgb[i].tl = m.tl.as<int32_t>();
     hgb[i].ql = m.ql.as<int2>();
     hgb[i].hq = m.hq.as<int2>();
     hgb[i].ctl = m.ctl.as<Ctl>();
@@ -1285,7 +1285,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
       int level = 0, cur_dir = kDirTD, max_level = 0, td = 0, bu = 0, err = 0;
       unsigned long long m_u = (unsigned long long)g->E, teps = 0, prev_changed = 0;
       while (true) {
-        CU(cudaMemcpyAsync(hpar, &gb.ctl->par[level & 1], sizeof(Par), cudaMemcpyDeviceToHost, s));
+        CU(cudaMemcpyAsync(hpar, par_at(gb.ctl, level), sizeof(Par), cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         const Par pr = *hpar;
         teps += pr.teps;
@@ -1312,7 +1312,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
           CU(cudaMemsetAsync(gb.planes + (size_t)pb * p.plane_stride, 0,
                              (size_t)p.plane_stride * 4, s));
         }
-        CU(cudaMemsetAsync(&gb.ctl->par[level & 1], 0, sizeof(Par), s));
+        CU(cudaMemsetAsync(par_at(gb.ctl, level), 0, sizeof(Par), s));
         CU(cudaMemsetAsync(&gb.ctl->qc[level & 1][0], 0, sizeof(int32_t) * 4, s));
         CU(DISPATCH_WORDS(rp.words, launch_plain_level, p, gb, grid, thr, level, cur_dir, s));
         launches += 2;

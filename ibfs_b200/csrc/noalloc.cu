@@ -26,7 +26,6 @@ namespace {
 
 constexpr size_t kScratchBytes = 64ull << 20;  // the fixed maximum
 constexpr int kMaxBatches = 16;
-constexpr int kLrecCap = 64;
 constexpr int kMaxSources = kMaxBatches * 256;
 
 // The scratch.  In host code `g_scratch` is only a stand-in symbol: its
@@ -86,13 +85,12 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   const size_t o_gb = off; off = align256(off + sizeof(GroupBufs));
   const size_t o_ctl = off; off = align256(off + sizeof(Ctl));
   const size_t o_brec = off; off = align256(off + sizeof(BatchRec) * kMaxBatches);
-  const size_t o_lrec = off; off = align256(off + sizeof(LevelRec) * kMaxBatches * kLrecCap);
   const size_t o_last = off; off = align256(off + vpad * words * 4);
   const size_t o_curr = off; off = align256(off + vpad * words * 4);
   const size_t o_chg = off; off = align256(off + 2 * nchg * 4);
   const size_t o_planes = off; off = align256(off + 8 * vpad * words * 4);
-  const size_t o_qs = off; off = align256(off + (size_t)V * 4);
-  const size_t o_qm = off; off = align256(off + (size_t)V * 4);
+  const size_t o_q = off; off = align256(off + (size_t)V * 4);
+  const size_t o_tl = off; off = align256(off + (size_t)V * 4);
   const size_t o_ql = off; off = align256(off + capl * 8);
   if (off > kScratchBytes) return IBFS_ERR_RANGE;  // graph too large for the fixed scratch
 
@@ -115,8 +113,8 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   gb.curr = reinterpret_cast<uint32_t*>(base + o_curr);
   gb.chg = reinterpret_cast<uint32_t*>(base + o_chg);
   gb.planes = reinterpret_cast<uint32_t*>(base + o_planes);
-  gb.qs = reinterpret_cast<int32_t*>(base + o_qs);
-  gb.qm = reinterpret_cast<int32_t*>(base + o_qm);
+  gb.q = reinterpret_cast<int32_t*>(base + o_q);
+  gb.tl = reinterpret_cast<int32_t*>(base + o_tl);
   gb.ql = reinterpret_cast<int2*>(base + o_ql);
   gb.hq = nullptr;
   gb.ctl = reinterpret_cast<Ctl*>(base + o_ctl);
@@ -165,8 +163,8 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   p.withhold = 0;
   p.groups = reinterpret_cast<GroupBufs*>(base + o_gb);
   p.brec = reinterpret_cast<BatchRec*>(base + o_brec);
-  p.lrec = reinterpret_cast<LevelRec*>(base + o_lrec);
-  p.lrec_cap = kLrecCap;
+  p.lrec = nullptr;  // no level records
+  p.lrec_cap = 0;
   p.vec_out = ((reinterpret_cast<uintptr_t>(depth_dev) & 3) == 0) ? 1 : 0;
   p.hub_t = INT32_MAX;  // no deferred hub chunks here: the sweep scans whole lists
   p.bu_filter = 0;

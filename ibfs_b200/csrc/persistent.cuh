@@ -19,7 +19,7 @@ namespace ibfs {
 // hence how many warps per SM hide the latency of the random gathers.
 template <int WORDS, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
-  __shared__ int s_dir, s_stop, s_err, s_maxl, s_dense;
+  __shared__ int s_dir, s_stop, s_err, s_maxl, s_thin;
   __shared__ int32_t s_rows[kMaxWords * 32];
   const int g = blockIdx.x / p.cpg;
   const Team t = make_team(blockIdx.x % p.cpg, p.cpg);
@@ -44,21 +44,22 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
     zero_words(gb.chg, 2 * p.chg_stride, t);
     load_rows(p, b, n_b, s_rows);
     if (lead) {
-      memset(&ctl->par[0], 0, sizeof(Par) * 2);
+      memset(&ctl->par[0], 0, sizeof(ctl->par));
       memset(&ctl->qc[0][0], 0, sizeof(ctl->qc));
     }
     BARRIER();
-    seed_phase<WORDS>(p, gb, p.src + k0, n_b, t);
+    seed_phase<WORDS, true>(p, gb, p.src + k0, n_b, t);
     BARRIER();
-    inspect_phase<WORDS, true>(p, gb, &ctl->par[0], n_b, 0, true, false, t);
+    inspect_phase<WORDS>(p, gb, &ctl->par[0], n_b, 0, true, true, ctl->qc[1], t);
     BARRIER();
     int level = 0, cur_dir = kDirTD, max_level = 0, td = 0, bu = 0;
     unsigned long long m_u = (unsigned long long)p.E, teps = 0, prev_changed = 0;
     unsigned long long t_lvl = global_ns(), t_mid = t_lvl;
     int err = 0;
+    bool have_q = true;  // the queues of the next level are built (by a thin inspect)
     while (true) {
       if (threadIdx.x == 0) {
-        const volatile Par* pr = &ctl->par[level & 1];
+        const volatile Par* pr = par_at(ctl, level);
         const unsigned long long changed = pr->changed, mf = pr->mf, cdeg = pr->cdeg;
         teps += pr->teps;
         m_u = m_u > cdeg ? m_u - cdeg : 0ull;
@@ -82,7 +83,9 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
             p.lrec[(size_t)b * p.lrec_cap + level] = r;
           }
           if (!stop) {
-            memset((void*)&ctl->par[(level + 1) & 1], 0, sizeof(Par));
+            // level-1's set becomes level+2's: no CTA reads it any more, and
+            // none writes it before the next barrier
+            memset((void*)par_at(ctl, level + 2), 0, sizeof(Par));
             ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
           }
         }
@@ -90,13 +93,13 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
         s_stop = stop;
         s_err = err;
         s_maxl = max_level;
-        s_dense = inspect_dense(mf, p.V) ? 1 : 0;
+        s_thin = mf <= kThinEdges ? 1 : 0;
       }
       __syncthreads();
       const int stop = s_stop;
       cur_dir = s_dir;
       err = s_err;
-      const bool dense = s_dense != 0;
+      const bool thin = s_thin != 0 && cur_dir == kDirTD;
       __syncthreads();
       if (stop) break;
       level++;
@@ -104,19 +107,21 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
       zero_plane_if_first(p, gb, level, t);
       if (cur_dir == kDirTD) {
         td++;
-        qbuild_phase(p, gb, level, ctl->qc[level & 1], t);
-        BARRIER();
-        td_phase<WORDS>(p, gb, level, ctl->qc[level & 1], t);
+        if (!have_q) {
+          qbuild_phase(p, gb, level, ctl->qc[level & 1], t);
+          BARRIER();
+        }
+        td_phase<WORDS>(p, gb, level, ctl->qc[level & 1], thin, t);
       } else {
         bu++;
         const bool filt =
-            bu_filter_level(p.bu_filter, __ldcg(&ctl->par[(level - 1) & 1].changed), p.V);
-        bu_phase<WORDS>(p, gb, level, ctl->par[(level - 1) & 1].fmask,
-                        &ctl->par[level & 1].hq_cnt, t, nullptr, 0, true, filt);
+            bu_filter_level(p.bu_filter, __ldcg(&par_at(ctl, level - 1)->changed), p.V);
+        bu_phase<WORDS>(p, gb, level, par_at(ctl, level - 1)->fmask,
+                        &par_at(ctl, level)->hq_cnt, t, nullptr, 0, true, filt);
         BARRIER();
-        if (__ldcg(&ctl->par[level & 1].hq_cnt) > 0) {  // same value in every CTA
-          bu_defer_phase<WORDS>(p, gb, level, ctl->par[(level - 1) & 1].fmask,
-                                &ctl->par[level & 1].hq_cnt, t, filt);
+        if (__ldcg(&par_at(ctl, level)->hq_cnt) > 0) {  // same value in every CTA
+          bu_defer_phase<WORDS>(p, gb, level, par_at(ctl, level - 1)->fmask,
+                                &par_at(ctl, level)->hq_cnt, t, filt);
           BARRIER();
         }
         if (lead) t_mid = global_ns();
@@ -126,8 +131,9 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
         BARRIER();
         if (lead) t_mid = global_ns();
       }
-      inspect_phase<WORDS, true>(p, gb, &ctl->par[level & 1], n_b, level,
-                                 level <= depth_limit(p.db), dense, t);
+      inspect_phase<WORDS>(p, gb, par_at(ctl, level), n_b, level, level <= depth_limit(p.db), thin,
+                           ctl->qc[(level + 1) & 1], t);
+      have_q = thin;
       BARRIER();
     }
     if (err) {
