@@ -82,12 +82,11 @@ struct LoopState {
 
 // Control block of one group (one batch at a time).  256-byte aligned.
 struct __align__(256) Ctl {
-  unsigned int bar_count;
-  unsigned int bar_gen;
+  unsigned int bar_count;  // barrier arrivals of the run so far
   int err;
-  int pad0;
+  int pad0[2];
   Par par[3];
-  int32_t qc[2][4];  // [consumer level parity][small, medium, large-chunks]
+  __align__(16) int32_t qc[2][4];  // [consumer level parity][small, medium, large-chunks]
   unsigned long long pad1[4];
   LoopState ls;
 };
@@ -312,13 +311,30 @@ __device__ __forceinline__ void ld_status_nc(const uint32_t* p, uint32_t (&x)[WO
   }
 }
 
+// Status read through L1 inside the persistent kernel, for a buffer that no
+// thread writes during the phase: the team barrier before the phase (release
+// by every CTA, acquire by every CTA, then a CTA barrier) makes the earlier
+// writes visible to ordinary cached loads.
+template <int WORDS>
+__device__ __forceinline__ void ld_status_ca(const uint32_t* p, uint32_t (&x)[WORDS]) {
+  if constexpr (WORDS == 1) {
+    x[0] = __ldca(p);
+  } else if constexpr (WORDS == 2) {
+    uint2 t = __ldca(reinterpret_cast<const uint2*>(p));
+    x[0] = t.x; x[1] = t.y;
+  } else {
+#pragma unroll
+    for (int q = 0; q < WORDS / 4; q++) {
+      uint4 t = __ldca(reinterpret_cast<const uint4*>(p) + q);
+      x[4 * q] = t.x; x[4 * q + 1] = t.y; x[4 * q + 2] = t.z; x[4 * q + 3] = t.w;
+    }
+  }
+}
+
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ int ld_volatile_i32(const int* p) {
   return *reinterpret_cast<const volatile int*>(p);
@@ -344,40 +360,38 @@ __host__ __device__ __forceinline__ int planes_for(int max_level) {
   return p;
 }
 
-// Bounded team barrier.  All waits end: after timeout_ns the waiting CTA
-// records IBFS_ERR_TIMEOUT (6) in ctl->err and every other CTA leaves on
-// seeing a non-zero err.  Returns false when the team must stop.
-static __device__ __noinline__ bool team_barrier(Ctl* ctl, unsigned nblocks,
+// Bounded team barrier.  Every CTA adds one to a counter that only grows
+// (the host zeroes it before a run) and waits for the barrier's own target
+// on that counter, so the last arrival releases the waiters directly: one
+// reduction and one polled line, instead of a returned atomic, a reset and a
+// release store.  All waits end: after timeout_ns the waiting CTA records
+// IBFS_ERR_TIMEOUT (6) in ctl->err, and the others leave on seeing it.
+// Returns false when the team must stop.
+static __device__ __noinline__ bool team_barrier(Ctl* ctl, unsigned nblocks, unsigned target,
                                                  unsigned long long timeout_ns,
                                                  bool withhold) {
   __shared__ int s_ok;
+  if (nblocks == 1 && !withhold) {  // a team of one CTA
+    __syncthreads();
+    return true;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
-    const unsigned gen = ld_acquire_u32(&ctl->bar_gen);
-    if (!withhold) {
-      __threadfence();
-      const unsigned prev = atomicAdd(&ctl->bar_count, 1u);
-      if (prev == nblocks - 1) {
-        atomicExch(&ctl->bar_count, 0u);
-        __threadfence();
-        st_release_u32(&ctl->bar_gen, gen + 1);
+    if (!withhold)
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
+    unsigned long long t0 = 0;
+    for (unsigned spin = 1; (int)(ld_acquire_u32(&ctl->bar_count) - target) < 0; spin++) {
+      if (spin & 63u) continue;
+      if (ld_volatile_i32(&ctl->err) != 0) { ok = 0; break; }
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > timeout_ns) {
+        atomicCAS(&ctl->err, 0, 6);
+        ok = 0;
+        break;
       }
     }
-    if (ld_acquire_u32(&ctl->bar_gen) == gen) {
-      const unsigned long long t0 = global_ns();
-      while (ld_acquire_u32(&ctl->bar_gen) == gen) {
-        if (ld_volatile_i32(&ctl->err) != 0) { ok = 0; break; }
-        if (global_ns() - t0 > timeout_ns) {
-          atomicCAS(&ctl->err, 0, 6);
-          ok = 0;
-          break;
-        }
-        __nanosleep(100);
-      }
-    }
-    __threadfence();
-    if (ld_volatile_i32(&ctl->err) != 0) ok = 0;
     s_ok = ok;
   }
   __syncthreads();
@@ -458,6 +472,15 @@ __device__ __forceinline__ void zero_words(uint32_t* p, long long nwords, const 
   uint4* q = reinterpret_cast<uint4*>(p);
   const uint4 z = make_uint4(0, 0, 0, 0);
   for (long long i = t.tid; i < nwords / 4; i += t.nthreads) __stcg(q + i, z);
+}
+
+// One warp zeroes a level's counters, a word per lane and step.  (A memset by
+// one thread became a chain of byte stores: 67 us for the three sets of a
+// batch, which was half of a small run.)
+__device__ __forceinline__ void zero_par(Par* par, int lane) {
+  static_assert(sizeof(Par) % 8 == 0, "whole words");
+  unsigned long long* q = reinterpret_cast<unsigned long long*>(par);
+  for (int i = lane; i < (int)(sizeof(Par) / 8); i += 32) q[i] = 0ull;
 }
 
 // ---------------------------------------------------------------------------
@@ -963,7 +986,8 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
                                        const int32_t* qc, const Team& t) {
   uint32_t* chg = chg_at(gb, p, level);
   int32_t* t_cnt = &par_at(gb.ctl, level)->t_cnt;
-  const int nS = __ldcg(qc + 0), nM = __ldcg(qc + 1), nL = __ldcg(qc + 2);
+  const int4 nq = __ldcg(reinterpret_cast<const int4*>(qc));  // small, medium, large chunks
+  const int nS = nq.x, nM = nq.y, nL = nq.z;
   if (STAGE && p.td_stage) {
     __shared__ __align__(128) int32_t s_col[2][kStageInts];
     __shared__ __align__(8) unsigned long long s_bar[2];
@@ -1213,7 +1237,9 @@ __device__ void bu_defer_phase(const Params& p, const GroupBufs& gb, int level,
 // planes and counters in bu_hub_epilogue.
 // Status of neighbour u for a bottom-up scan: from the CTA's shared-memory
 // copy of the hubs' statuses when u is one of the first hk vertices, else
-// from `last` (through L1 when NC: `last` is read-only during a fused pass).
+// from `last`, which no thread writes during the pass (through L1: the
+// read-only path when the pass is a kernel of its own (NC), ordinary cached
+// loads in the persistent kernel).
 template <int WORDS, int HK, bool NC>
 __device__ __forceinline__ void ld_nbr(const uint32_t* last, const uint32_t* s_hub, long long hk,
                                        int32_t u, uint32_t (&x)[WORDS]) {
@@ -1231,7 +1257,52 @@ __device__ __forceinline__ void ld_nbr(const uint32_t* last, const uint32_t* s_h
     return;
   }
   if constexpr (NC) ld_status_nc<WORDS>(last + (size_t)u * WORDS, x);
-  else ld_status<WORDS>(last + (size_t)u * WORDS, x);
+  else ld_status_ca<WORDS>(last + (size_t)u * WORDS, x);
+}
+
+// A warp ORs the statuses of the neighbours [e0, e_lim) of one vertex into a
+// (the same value in every lane) until no bit of fm is missing; returns
+// whether one still is.  The first step reads 32 neighbours (the highest
+// degrees, which usually cover the bits), the later ones 128: a long scan is
+// a chain of steps, and with 4 gathers per lane in flight it has a quarter
+// of them.
+template <int WORDS, int HK, bool NC, bool RO>
+__device__ __forceinline__ bool warp_scan(const Params& p, const GroupBufs& gb,
+                                          const uint32_t* s_hub, long long hk,
+                                          const uint32_t* front, bool filt, int lane,
+                                          long long e0, long long e_lim,
+                                          const uint32_t (&fm)[WORDS], uint32_t (&a)[WORDS]) {
+  // gathers in flight per lane; the kernel of its own, whose 42 registers
+  // already spill, keeps one (its warps hide the chain)
+  constexpr int D = RO ? 1 : WORDS <= 4 ? 4 : 2;
+  bool miss = true;
+  int width = 32;
+  for (long long e = e0; e < e_lim;) {
+    uint32_t x[D][WORDS];
+#pragma unroll
+    for (int i = 0; i < D; i++) {
+#pragma unroll
+      for (int k = 0; k < WORDS; k++) x[i][k] = 0;
+      const long long ei = e + lane + 32 * i;
+      if (32 * i < width && ei < e_lim) {
+        const int32_t u = __ldg(p.col + ei);
+        if (!filt || in_front<RO>(front, u)) ld_nbr<WORDS, HK, NC>(gb.last, s_hub, hk, u, x[i]);
+      }
+    }
+    miss = false;
+#pragma unroll
+    for (int k = 0; k < WORDS; k++) {
+      uint32_t r = x[0][k];
+#pragma unroll
+      for (int i = 1; i < D; i++) r |= x[i][k];
+      a[k] |= __reduce_or_sync(0xFFFFFFFFu, r);
+      miss |= (fm[k] & ~a[k]) != 0u;
+    }
+    if (!miss) break;
+    e += width;
+    width = 32 * D;
+  }
+  return miss;
 }
 
 // smask (device loop, sparse-source levels): bits pushed top-down after this
@@ -1295,24 +1366,8 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
     bool defer = false;
     if (need) {
       const long long e_lim = (e1 - e0 > p.hub_t) ? e0 + p.hub_t : e1;
-      bool miss = true;
-      for (long long e = e0; e < e_lim; e += 32) {
-        uint32_t x[WORDS];
-#pragma unroll
-        for (int k = 0; k < WORDS; k++) x[k] = 0;
-        if (e + lane < e_lim) {
-          const int32_t u = p.col[e + lane];
-          if (!filt || in_front<RO>(front, u))
-            ld_nbr<WORDS, HK, NC>(gb.last, s_hub, hk, u, x);
-        }
-        miss = false;
-#pragma unroll
-        for (int k = 0; k < WORDS; k++) {
-          a[k] |= __reduce_or_sync(0xFFFFFFFFu, x[k]);
-          miss |= (fm[k] & ~a[k]) != 0u;
-        }
-        if (!miss) break;
-      }
+      const bool miss =
+          warp_scan<WORDS, HK, NC, RO>(p, gb, s_hub, hk, front, filt, lane, e0, e_lim, fm, a);
       defer = miss && e_lim < e1;
       if (defer && lane == 0) {
         const int nch = (int)((e1 - e_lim + kHubChunk - 1) / kHubChunk);
@@ -1475,24 +1530,8 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       // still missing frontier bits is deferred to bu_defer_phase
       // (the limit counts from the list's start, as bu_defer_phase does)
       const long long e_lim = (e1 - e0 > p.hub_t) ? e0 + p.hub_t : e1;
-      bool miss = true;
-      for (long long e = es; e < e_lim; e += 32) {
-        uint32_t x[WORDS];
-#pragma unroll
-        for (int k = 0; k < WORDS; k++) x[k] = 0;
-        if (e + lane < e_lim) {
-          const int32_t u = p.col[e + lane];
-          if (!filt || in_front<RO>(front, u))
-            ld_nbr<WORDS, HK, NC>(gb.last, s_hub, hk, u, x);
-        }
-        miss = false;
-#pragma unroll
-        for (int k = 0; k < WORDS; k++) {
-          a[k] |= __reduce_or_sync(0xFFFFFFFFu, x[k]);
-          miss |= (fm[k] & ~a[k]) != 0u;
-        }
-        if (!miss) break;
-      }
+      const bool miss =
+          warp_scan<WORDS, HK, NC, RO>(p, gb, s_hub, hk, front, filt, lane, es, e_lim, fm, a);
       const bool defer = miss && e_lim < e1;
       if (defer && lane == 0) {
         const int nch = (int)((e1 - e_lim + kHubChunk - 1) / kHubChunk);

@@ -196,10 +196,12 @@ __global__ void __launch_bounds__(512) k_dl_batch_init(Params p, int g, CondH h_
   zero_words(gb.last, zv * WORDS, t);
   zero_words(gb.curr, zv * WORDS, t);
   zero_words(gb.chg, 2 * p.chg_stride, t);
+  if (t.warp == 0) {
+    for (int i = 0; i < 3; i++) zero_par(&gb.ctl->par[i], t.lane);
+    if (t.lane < 8) (&gb.ctl->qc[0][0])[t.lane] = 0;
+  }
   if (t.tid == 0) {
     Ctl* ctl = gb.ctl;
-    memset(&ctl->par[0], 0, sizeof(ctl->par));
-    memset(&ctl->qc[0][0], 0, sizeof(ctl->qc));
     LoopState& ls = ctl->ls;
     ls.level = 0;
     ls.dir = kDirTD;
@@ -243,10 +245,13 @@ __global__ void DL_INSPECT_BOUNDS k_dl_inspect(Params p, int g, CondH, CondH) {
 // h_level keeps the level loop running, h_dir selects the expand body
 // (0 top-down, 1 bottom-up, 2 none: the loop ends).
 __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  if (blockIdx.x != 0) return;
   Ctl* ctl = p.groups[g].ctl;
   LoopState& ls = ctl->ls;
   const int level = ls.level, b = ls.batch;
+  __syncwarp();  // every lane has read the level that lane 0 advances
+  zero_par(par_at(ctl, level + 1), threadIdx.x);
+  if (threadIdx.x != 0) return;
   // a fused bottom-up level left its statuses in the other buffer
   const bool was_bu = IBFS_DL_FUSED_BU && level > 0 && ls.dir == kDirBU;
   if (was_bu) ls.flip ^= 1;
@@ -279,7 +284,6 @@ __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
   ls.t_lvl = t_now;
   ls.err = err;
   if (!stop) {
-    memset((void*)par_at(ctl, level + 1), 0, sizeof(Par));
     ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
     // a thin level left the next level's queues behind
     ls.have_q = (nd == kDirTD && ls.thin && ls.dir == kDirTD) ? 1 : 0;

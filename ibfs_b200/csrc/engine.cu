@@ -265,6 +265,20 @@ static size_t group_bytes(int64_t V, int64_t E, int words, int C, int db, int lr
 // arguments below).
 static const int kOccThreads[4] = {512, 256, 256, 512};
 
+// CTAs of a persistent team for a graph of E edges: 512 threads per 12288
+// edges, at least 32 CTAs of 512, and more than one per SM only when every
+// SM gets its full share -- a barrier of a thin level costs more with every
+// CTA that has nothing to do, and SMs that hold two CTAs while others hold
+// one only unbalance the phases.  One run, 32 / 64 / 148 / 296 CTAs: R-MAT
+// scale 12, 1 source 79 / 78 / 82 / 97 us; scale 16, 128 sources 283 / 215 /
+// 187 / 220 us; scale 18, 128 sources 1068 / 617 / 384 / 371 us; grid strip
+// 256 x 1024 28.6 / 23.6 / 23.8 / 31.1 ms.
+int team_ctas(int64_t E, int sms, int total_ctas, int threads) {
+  const int64_t want = std::max<int64_t>(E / 12288, 32) * 512 / threads;
+  if (want >= total_ctas) return total_ctas;
+  return (int)std::min<int64_t>(want, std::min(total_ctas, sms * 512 / threads));
+}
+
 static const void* persistent_for(int words, int level = 0) {
   switch (words) {
     case 1: return persistent_fn_w32(level);
@@ -928,6 +942,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     G = std::max(1, std::min(G, std::min(rp.nbatches, total_ctas)));
     rp.G = G;
     rp.cpg = total_ctas / G;
+    if (!o.ctas_per_sm) rp.cpg = std::min(rp.cpg, team_ctas(g->E, g->sms, total_ctas, rp.threads));
     rp.grid = rp.cpg * G;
   } else if (devloop) {
     // concurrent batches are parallel branches of the graph; each kernel is

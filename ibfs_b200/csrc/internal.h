@@ -75,6 +75,7 @@ ibfs_status run_rows(ibfs_graph* g, const int32_t* src, const int32_t* rows, int
 int graph_device(const ibfs_graph* g);
 const int64_t* graph_host_beg(const ibfs_graph* g);
 const int32_t* graph_host_col(const ibfs_graph* g);
+int team_ctas(int64_t E, int sms, int total_ctas, int threads);
 int graph_sms(const ibfs_graph* g);
 int64_t graph_defer_cap(const ibfs_graph* g);
 const int32_t* graph_new_of_old(const ibfs_graph* g);  // caller id -> internal id (host)

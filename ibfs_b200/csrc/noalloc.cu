@@ -147,7 +147,7 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   p.C = width;
   p.nbatches = nbatches;
   p.G = 1;
-  p.cpg = sms * per_sm;
+  p.cpg = team_ctas(E, sms, sms * per_sm, threads);
   p.db = 1;
   p.layout = IBFS_LAYOUT_VERTEX_MAJOR;
   p.out = static_cast<uint8_t*>(depth_dev);

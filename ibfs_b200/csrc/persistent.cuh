@@ -6,7 +6,6 @@
 // (persistent_w32/64/128/256.cu), which exports the kernels' addresses per
 // occupancy level through persistent_fn_w<W>().
 #pragma once
-#include <cstring>
 
 #include <cuda_runtime.h>
 
@@ -23,41 +22,49 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
   __shared__ int32_t s_rows[kMaxWords * 32];
   const int g = blockIdx.x / p.cpg;
   const Team t = make_team(blockIdx.x % p.cpg, p.cpg);
-  const GroupBufs gb = p.groups[g];
+  GroupBufs gb = p.groups[g];  // last and curr swap roles after bottom-up levels
   Ctl* ctl = gb.ctl;
   const unsigned nb = (unsigned)p.cpg;
   const bool lead = (t.block == 0 && threadIdx.x == 0);
   bool withhold = p.withhold && t.block == 0 && g == 0;
   const long long vpad = (p.V + 31) & ~31LL;
 
+  unsigned bar_target = 0;
 #define BARRIER()                                                   \
   do {                                                              \
-    if (!team_barrier(ctl, nb, p.timeout_ns, withhold)) return;     \
+    bar_target += nb;                                               \
+    if (!team_barrier(ctl, nb, bar_target, p.timeout_ns, withhold)) return; \
     withhold = false;                                               \
   } while (0)
 
   for (int b = g; b < p.nbatches; b += p.G) {
     const long long k0 = (long long)b * p.C;
     const int n_b = (int)min((long long)p.C, p.n_total - k0);
+    unsigned long long t_lvl = global_ns(), t_mid = t_lvl;
     zero_words(gb.last, vpad * WORDS, t);
     zero_words(gb.curr, vpad * WORDS, t);
     zero_words(gb.chg, 2 * p.chg_stride, t);
     load_rows(p, b, n_b, s_rows);
-    if (lead) {
-      memset(&ctl->par[0], 0, sizeof(ctl->par));
-      memset(&ctl->qc[0][0], 0, sizeof(ctl->qc));
+    if (t.block == 0 && threadIdx.x < 32) {
+      for (int i = 0; i < 3; i++) zero_par(&ctl->par[i], t.lane);
+      if (threadIdx.x < 8) (&ctl->qc[0][0])[threadIdx.x] = 0;
     }
     BARRIER();
     seed_phase<WORDS, true>(p, gb, p.src + k0, n_b, t);
     BARRIER();
+    if (lead) t_mid = global_ns();
     inspect_phase<WORDS>(p, gb, &ctl->par[0], n_b, 0, true, true, ctl->qc[1], t);
     BARRIER();
     int level = 0, cur_dir = kDirTD, max_level = 0, td = 0, bu = 0;
     unsigned long long m_u = (unsigned long long)p.E, teps = 0, prev_changed = 0;
-    unsigned long long t_lvl = global_ns(), t_mid = t_lvl;
     int err = 0;
-    bool have_q = true;  // the queues of the next level are built (by a thin inspect)
+    bool have_q = true;     // the queues of the next level are built (by a thin inspect)
+    bool after_bu = false;  // the level before was bottom-up: `curr` is one level behind
     while (true) {
+      // level-1's counters become level+2's: no CTA reads them any more, and
+      // none adds to them before the next barrier
+      if (t.block == 0 && threadIdx.x >= 32 && threadIdx.x < 64)
+        zero_par(par_at(ctl, level + 2), t.lane);
       if (threadIdx.x == 0) {
         const volatile Par* pr = par_at(ctl, level);
         const unsigned long long changed = pr->changed, mf = pr->mf, cdeg = pr->cdeg;
@@ -82,12 +89,7 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
             t_lvl = t_now;
             p.lrec[(size_t)b * p.lrec_cap + level] = r;
           }
-          if (!stop) {
-            // level-1's set becomes level+2's: no CTA reads it any more, and
-            // none writes it before the next barrier
-            memset((void*)par_at(ctl, level + 2), 0, sizeof(Par));
-            ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
-          }
+          if (!stop) ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
         }
         s_dir = nd;
         s_stop = stop;
@@ -103,37 +105,49 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
       __syncthreads();
       if (stop) break;
       level++;
-      bool continue_inspect = false;
-      zero_plane_if_first(p, gb, level, t);
+      const bool depth_ok = level <= depth_limit(p.db);
       if (cur_dir == kDirTD) {
         td++;
+        zero_plane_if_first(p, gb, level, t);
         if (!have_q) {
-          qbuild_phase(p, gb, level, ctl->qc[level & 1], t);
+          qbuild_phase<WORDS>(p, gb, level, ctl->qc[level & 1], t, after_bu);
           BARRIER();
         }
         td_phase<WORDS>(p, gb, level, ctl->qc[level & 1], thin, t);
+        BARRIER();
+        if (lead) t_mid = global_ns();
+        inspect_phase<WORDS>(p, gb, par_at(ctl, level), n_b, level, depth_ok, thin,
+                             ctl->qc[(level + 1) & 1], t);
+        have_q = thin;
+        after_bu = false;
       } else {
+        // Fused with its inspect work, as in the device loop: the pass writes
+        // every vertex's new status to `curr`, and the buffers swap roles.
         bu++;
-        const bool filt =
-            bu_filter_level(p.bu_filter, __ldcg(&par_at(ctl, level - 1)->changed), p.V);
-        bu_phase<WORDS>(p, gb, level, par_at(ctl, level - 1)->fmask,
-                        &par_at(ctl, level)->hq_cnt, t, nullptr, 0, true, filt);
+        Par* par = par_at(ctl, level);
+        const Par* prev = par_at(ctl, level - 1);
+        const bool filt = bu_filter_level(p.bu_filter, __ldcg(&prev->changed), p.V);
+        // the level-(L+1) bitmap is the buffer of level L-1's, which only the
+        // filter reads
+        if (!filt) zero_words(chg_at(gb, p, level + 1), p.chg_stride, t);
+        bu_phase<WORDS, true, false>(p, gb, level, prev->fmask, &par->hq_cnt, t, par, n_b,
+                                     depth_ok, filt);
         BARRIER();
-        if (__ldcg(&par_at(ctl, level)->hq_cnt) > 0) {  // same value in every CTA
-          bu_defer_phase<WORDS>(p, gb, level, par_at(ctl, level - 1)->fmask,
-                                &par_at(ctl, level)->hq_cnt, t, filt);
+        if (lead) t_mid = global_ns();
+        if (__ldcg(&par->hq_cnt) > 0) {  // same value in every CTA
+          bu_defer_phase<WORDS>(p, gb, level, prev->fmask, &par->hq_cnt, t, filt);
           BARRIER();
+          bu_hub_epilogue<WORDS>(p, gb, par, n_b, level, depth_ok, t, !filt);
+        } else if (filt) {
+          zero_words(chg_at(gb, p, level + 1), p.chg_stride, t);
         }
-        if (lead) t_mid = global_ns();
-        continue_inspect = true;
+        uint32_t* x = gb.last;
+        gb.last = gb.curr;
+        gb.curr = x;
+        have_q = false;
+        after_bu = true;
+        if (!filt && __ldcg(&par->hq_cnt) == 0) continue;  // nothing since the barrier
       }
-      if (!continue_inspect) {
-        BARRIER();
-        if (lead) t_mid = global_ns();
-      }
-      inspect_phase<WORDS>(p, gb, par_at(ctl, level), n_b, level, level <= depth_limit(p.db), thin,
-                           ctl->qc[(level + 1) & 1], t);
-      have_q = thin;
       BARRIER();
     }
     if (err) {
