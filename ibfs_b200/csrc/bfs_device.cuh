@@ -50,8 +50,6 @@ struct Par {
   int32_t hq_cnt;              // deferred bottom-up hub chunks of this level
   int32_t pq_cnt;              // queued sparse-source push chunks of this level
   int32_t t_cnt;               // vertices in the touched list of this level
-  uint32_t scnt[kMaxWords * 32];  // per source: vertices it reached at the
-                                  // previous level (sparse_count_phase)
 };
 
 // State of the level loop when it runs as kernels inside a CUDA graph (the
@@ -115,7 +113,9 @@ struct GroupBufs {
   uint32_t* planes;  // depth bit-planes, plane b at b*plane_stride words
   int32_t* q;        // [V] frontier queue: small vertices from the front, medium
                      // ones from the back (a vertex is in one class only)
-  int32_t* tl;       // [V] touched list of a thin top-down level
+  int32_t* tl;       // [V] touched list of a thin top-down level; on a bottom-up
+                     // level that picks sparse sources, its first W entries
+                     // count each source's previous frontier
   int2* ql;
   int2* hq;          // deferred bottom-up hub chunks (v, chunk)
   Ctl* ctl;
@@ -461,10 +461,10 @@ __device__ __forceinline__ void scnt_begin(uint32_t* s_cnt) {
   __syncthreads();
 }
 template <int WORDS>
-__device__ __forceinline__ void scnt_flush(const uint32_t* s_cnt, Par* par) {
+__device__ __forceinline__ void scnt_flush(const uint32_t* s_cnt, int32_t* dst) {
   __syncthreads();
   for (int i = threadIdx.x; i < WORDS * 32; i += blockDim.x)
-    if (s_cnt[i]) atomicAdd(&par->scnt[i], s_cnt[i]);
+    if (s_cnt[i]) atomicAdd(&dst[i], (int)s_cnt[i]);
 }
 
 __device__ __forceinline__ void zero_words(uint32_t* p, long long nwords, const Team& t) {
@@ -1729,7 +1729,7 @@ __device__ __forceinline__ bool gained_at(const Params& p, const GroupBufs& gb, 
 }
 
 template <int WORDS>
-__device__ void sparse_count_phase(const Params& p, const GroupBufs& gb, Par* par, int level,
+__device__ void sparse_count_phase(const Params& p, const GroupBufs& gb, int level,
                                    const Team& t) {
   __shared__ uint32_t s_scnt[kMaxWords * 32];
   scnt_begin(s_scnt);
@@ -1750,7 +1750,7 @@ __device__ void sparse_count_phase(const Params& p, const GroupBufs& gb, Par* pa
       }
     }
   }
-  scnt_flush<WORDS>(s_scnt, par);
+  scnt_flush<WORDS>(s_scnt, gb.tl);
 }
 
 struct PushAcc {

@@ -251,6 +251,8 @@ __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
   const int level = ls.level, b = ls.batch;
   __syncwarp();  // every lane has read the level that lane 0 advances
   zero_par(par_at(ctl, level + 1), threadIdx.x);
+  if (p.sparse_div > 0)  // the level's source counts, if it picks sparse sources
+    for (int i = threadIdx.x; i < kMaxWords * 32; i += 32) p.groups[g].tl[i] = 0;
   if (threadIdx.x != 0) return;
   // a fused bottom-up level left its statuses in the other buffer
   const bool was_bu = IBFS_DL_FUSED_BU && level > 0 && ls.dir == kDirBU;
@@ -366,7 +368,7 @@ __global__ void __launch_bounds__(512) k_dl_sparse_count(Params p, int g, CondH,
   Ctl* ctl = gb.ctl;
   if (!ctl->ls.sparse_try) return;  // uniform
   const int level = ctl->ls.level;
-  sparse_count_phase<WORDS>(p, gb, par_at(ctl, level), level, make_team(blockIdx.x, gridDim.x));
+  sparse_count_phase<WORDS>(p, gb, level, make_team(blockIdx.x, gridDim.x));
 }
 
 __global__ void k_dl_sparse_decide(Params p, int g, CondH, CondH) {
@@ -374,15 +376,15 @@ __global__ void k_dl_sparse_decide(Params p, int g, CondH, CondH) {
   Ctl* ctl = p.groups[g].ctl;
   LoopState& ls = ctl->ls;
   if (!ls.sparse_try) return;
-  const Par& pr = *par_at(ctl, ls.level);
+  const int32_t* scnt = p.groups[g].tl;
   const int nsrc = ls.nb;
   unsigned long long tot = 0;
-  for (int i = 0; i < nsrc; i++) tot += pr.scnt[i];
+  for (int i = 0; i < nsrc; i++) tot += (unsigned long long)scnt[i];
   uint32_t sm[kMaxWords];
 #pragma unroll
   for (int k = 0; k < kMaxWords; k++) sm[k] = 0u;
   for (int i = 0; i < nsrc; i++) {
-    const unsigned long long c = pr.scnt[i];
+    const unsigned long long c = (unsigned long long)scnt[i];
     if (c > 0 && c * (unsigned long long)p.sparse_div * (unsigned long long)nsrc < tot)
       sm[i >> 5] |= 1u << (i & 31);
   }

@@ -167,10 +167,10 @@ struct PinBuf {
 };
 
 struct GroupMem {
-  DevBuf last, curr, chg, q, tl, ql, hq, ctl, planes;
+  DevBuf last, curr, chg, q, tl, ql, hq, planes;
   void release() {
     last.release(); curr.release(); chg.release(); q.release();
-    tl.release(); ql.release(); hq.release(); ctl.release(); planes.release();
+    tl.release(); ql.release(); hq.release(); planes.release();
   }
 };
 
@@ -206,8 +206,11 @@ struct ibfs_graph {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // workspace
   std::vector<GroupMem> groups;
-  DevBuf d_groups, d_src, d_outrow, d_brec, d_lrec, d_out;
-  PinBuf h_src, h_outrow, h_brec, h_lrec, h_par;
+  // A run's small inputs and results live in one block, staged in pinned host
+  // memory at the same offsets (RunBlock): one copy in, one copy out.
+  DevBuf d_run, d_lrec, d_out;
+  PinBuf h_run, h_lrec, h_par;
+  int occ[4][4] = {};   // CTAs per SM of the persistent kernel by width and occupancy level
   GraphCache gcache;
   // depth sink of host-buffer runs, and the device loop's per-batch done
   // flags in mapped host memory (h_done; d_done is their device address)
@@ -325,6 +328,29 @@ static cudaError_t launch_plain_output(const Params& p, const GroupBufs& gb, int
   return cudaGetLastError();
 }
 
+// Byte offsets inside the run block: group table, control blocks, batch
+// records, sources, output rows.  The capacities are powers of two, so that the
+// addresses (baked into cached CUDA graphs) stay put across runs of similar
+// size.
+struct RunBlock {
+  size_t groups, ctl, brec, src, row, bytes;
+  RunBlock(int G, int nbatches, int64_t n) {
+    auto up = [](int64_t x, int64_t lo) {
+      int64_t r = lo;
+      while (r < x) r <<= 1;
+      return (size_t)r;
+    };
+    auto a256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t gc = up(G, 4), bc = up(nbatches, 64), nc = up(n, 256);
+    groups = 0;
+    ctl = a256(sizeof(GroupBufs) * gc);
+    brec = a256(ctl + sizeof(Ctl) * gc);
+    src = a256(brec + sizeof(BatchRec) * bc);
+    row = src + sizeof(int32_t) * nc;
+    bytes = row + sizeof(int32_t) * nc;
+  }
+};
+
 struct RunPlan {
   int words, C, nbatches, G, cpg, threads, grid, db;
   size_t smem;
@@ -349,10 +375,9 @@ static ibfs_status ensure_workspace(ibfs_graph* g, const RunPlan& rp, const ibfs
     if ((s = m.planes.ensure((size_t)(rp.db == 1 ? 8 : 16) * vpad * rp.words * 4)) != IBFS_OK)
       return s;
     if ((s = m.q.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
-    if ((s = m.tl.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
+    if ((s = m.tl.ensure((size_t)std::max<int64_t>(g->V, kMaxWords * 32) * 4)) != IBFS_OK) return s;
     if ((s = m.ql.ensure(capl * 8)) != IBFS_OK) return s;
     if ((s = m.hq.ensure((size_t)g->defer_cap * 8)) != IBFS_OK) return s;
-    if ((s = m.ctl.ensure(sizeof(Ctl))) != IBFS_OK) return s;
   }
   return IBFS_OK;
 }
@@ -655,15 +680,10 @@ static void destroy_graph(ibfs_graph* g) {
   g->vmap.release();
   g->gbin.release();
   g->gbkeys.release();
-  g->d_groups.release();
-  g->d_src.release();
-  g->d_outrow.release();
-  g->d_brec.release();
+  g->d_run.release();
   g->d_lrec.release();
   g->d_out.release();
-  g->h_src.release();
-  g->h_outrow.release();
-  g->h_brec.release();
+  g->h_run.release();
   g->h_lrec.release();
   g->h_par.release();
   g->sink.release();
@@ -884,15 +904,18 @@ extern "C" ibfs_status ibfs_run(ibfs_graph* g, const int32_t* src_host, int64_t 
 }
 
 // IBFS_MODE_AUTO: small graphs (one batch's status words within 32 MB, a
-// few levels of short kernels) run the persistent kernel from a CUDA graph,
-// where the device loop's per-kernel launch costs would dominate; larger
-// ones run the device loop.
+// few levels of short kernels) run the persistent kernel, where the device
+// loop's per-kernel launch costs would dominate; larger ones run the device
+// loop.  The persistent run is one copy in, one launch, one copy out, issued
+// directly: a captured graph (use_graph = 1) has the output pointer and the
+// source count baked in, so every new buffer would pay a capture and an
+// instantiation (R-MAT scale 12, 1 source, three output buffers in turn: 305 us
+// per call captured, 134 us direct).
 static ibfs_opts resolve_mode(const ibfs_graph* g, const ibfs_opts& in) {
   ibfs_opts o = in;
   if (o.mode == IBFS_MODE_AUTO) {
     const bool small = (double)g->V * (o.width / 8) <= 32.0 * 1024 * 1024;
     o.mode = small ? IBFS_MODE_PERSISTENT : IBFS_MODE_DEVICE_LOOP;
-    if (small && !o.debug_withhold) o.use_graph = 1;
   }
   return o;
 }
@@ -918,9 +941,15 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   const bool devloop = o.mode == IBFS_MODE_DEVICE_LOOP;
   // grid sizing
   int occ = 0;
-  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_for(rp.words, occ_level), rp.threads,
-                                                   rp.smem));
-  if (occ < 1) return IBFS_ERR_UNSUPPORTED;
+  int& occ_known = g->occ[rp.words == 8 ? 3 : rp.words / 2][occ_level];
+  if (persistent && occ_known) {
+    occ = occ_known;
+  } else {
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, persistent_for(rp.words, occ_level),
+                                                     rp.threads, rp.smem));
+    if (occ < 1) return IBFS_ERR_UNSUPPORTED;
+    if (persistent) occ_known = occ;
+  }
   int per_sm = o.ctas_per_sm ? std::min(o.ctas_per_sm, occ) : occ;
   const int total_ctas = g->sms * per_sm;
   if (persistent) {
@@ -977,10 +1006,17 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   }
   const bool dev_gb = o.groupby == 2 && !rows_in;
   ibfs_status bs;
-  if ((bs = g->h_src.ensure(sizeof(int32_t) * n)) != IBFS_OK) return bs;
-  if ((bs = g->h_outrow.ensure(sizeof(int32_t) * n)) != IBFS_OK) return bs;
-  if ((bs = g->d_src.ensure_pow2(sizeof(int32_t) * n)) != IBFS_OK) return bs;
-  if ((bs = g->d_outrow.ensure_pow2(sizeof(int32_t) * n)) != IBFS_OK) return bs;
+  const RunBlock rb(rp.G, rp.nbatches, n);
+  if ((bs = g->h_run.ensure(rb.bytes)) != IBFS_OK) return bs;
+  if ((bs = g->d_run.ensure(rb.bytes)) != IBFS_OK) return bs;
+  uint8_t* const hrun = g->h_run.as<uint8_t>();
+  uint8_t* const drun = g->d_run.as<uint8_t>();
+  int32_t* const hsrc = reinterpret_cast<int32_t*>(hrun + rb.src);
+  int32_t* const hrow = reinterpret_cast<int32_t*>(hrun + rb.row);
+  int32_t* const dsrc = reinterpret_cast<int32_t*>(drun + rb.src);
+  int32_t* const drow = reinterpret_cast<int32_t*>(drun + rb.row);
+  Ctl* const hctl = reinterpret_cast<Ctl*>(hrun + rb.ctl);
+  BatchRec* const hbrec = reinterpret_cast<BatchRec*>(hrun + rb.brec);
   int64_t gb_launches = 0;
   if (dev_gb) {
     const int64_t npad = groupby_dev_pad(n);
@@ -990,28 +1026,29 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     while ((1LL << lg) < npad) lg++;
     gb_launches = 2 + (npad <= 4096 ? 1 : (int64_t)lg * (lg + 1) / 2);
   }
-  // sources and output rows to the device: as ordered on the host, or in the
-  // caller's order and regrouped there
-  auto upload_sources = [&](cudaStream_t cs) -> ibfs_status {
+  // the run block to the device; with the device GroupBy the sources go to
+  // its input in the caller's order and are regrouped there
+  auto upload = [&](cudaStream_t cs) -> ibfs_status {
+    CU(cudaMemcpyAsync(drun, hrun, dev_gb ? rb.src : rb.row + sizeof(int32_t) * n,
+                       cudaMemcpyHostToDevice, cs));
     if (dev_gb) {
-      CU(cudaMemcpyAsync(g->gbin.p, g->h_src.p, sizeof(int32_t) * n, cudaMemcpyHostToDevice, cs));
+      CU(cudaMemcpyAsync(g->gbin.p, hsrc, sizeof(int32_t) * n, cudaMemcpyHostToDevice, cs));
       CU(groupby_dev_run(g->gbhub.as<int32_t>(), g->gbin.as<int32_t>(), n,
-                         g->gbkeys.as<unsigned long long>(), g->d_src.as<int32_t>(),
-                         g->d_outrow.as<int32_t>(), cs, g->vmap.as<int32_t>()));
-    } else {
-      CU(cudaMemcpyAsync(g->d_src.p, g->h_src.p, sizeof(int32_t) * n, cudaMemcpyHostToDevice, cs));
-      CU(cudaMemcpyAsync(g->d_outrow.p, g->h_outrow.p, sizeof(int32_t) * n,
-                         cudaMemcpyHostToDevice, cs));
+                         g->gbkeys.as<unsigned long long>(), dsrc, drow, cs,
+                         g->vmap.as<int32_t>()));
     }
     return IBFS_OK;
   };
-  if ((bs = g->d_brec.ensure_pow2(sizeof(BatchRec) * rp.nbatches)) != IBFS_OK) return bs;
-  if ((bs = g->h_brec.ensure(sizeof(BatchRec) * rp.nbatches)) != IBFS_OK) return bs;
+  // the control blocks and the batch records back, behind the traversal
+  auto download = [&](cudaStream_t cs) -> ibfs_status {
+    CU(cudaMemcpyAsync(hctl, drun + rb.ctl, rb.brec - rb.ctl + sizeof(BatchRec) * rp.nbatches,
+                       cudaMemcpyDeviceToHost, cs));
+    return IBFS_OK;
+  };
   if ((bs = g->d_lrec.ensure_pow2(sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap)) != IBFS_OK)
     return bs;
   if ((bs = g->h_lrec.ensure(sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap)) != IBFS_OK) return bs;
-  if ((bs = g->d_groups.ensure(sizeof(GroupBufs) * rp.G)) != IBFS_OK) return bs;
-  if ((bs = g->h_par.ensure(sizeof(Ctl) * rp.G + sizeof(GroupBufs) * rp.G)) != IBFS_OK) return bs;
+  if ((bs = g->h_par.ensure(sizeof(Par))) != IBFS_OK) return bs;
   const size_t out_bytes = (size_t)n * (size_t)g->V * db;
   uint8_t* dout = nullptr;
   if (rp.host_out) {
@@ -1029,13 +1066,13 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   {
     // sources in the graph's internal order (the device GroupBy renames its
     // output itself; it takes the caller's ids)
-    int32_t* hs = g->h_src.as<int32_t>();
-    if (dev_gb) std::memcpy(hs, ord.data(), sizeof(int32_t) * n);
+    if (dev_gb) std::memcpy(hsrc, ord.data(), sizeof(int32_t) * n);
     else
-      for (int64_t k = 0; k < n; k++) hs[k] = g->new_of_old[(size_t)ord[(size_t)k]];
+      for (int64_t k = 0; k < n; k++) hsrc[k] = g->new_of_old[(size_t)ord[(size_t)k]];
   }
-  std::memcpy(g->h_outrow.p, row.data(), sizeof(int32_t) * n);
-  GroupBufs* hgb = reinterpret_cast<GroupBufs*>(g->h_par.as<uint8_t>() + sizeof(Ctl) * rp.G);
+  std::memcpy(hrow, row.data(), sizeof(int32_t) * n);
+  std::memset(hctl, 0, rb.brec - rb.ctl + sizeof(BatchRec) * rp.nbatches);
+  GroupBufs* hgb = reinterpret_cast<GroupBufs*>(hrun + rb.groups);
   for (int i = 0; i < rp.G; i++) {
     GroupMem& m = g->groups[i];
     hgb[i].last = m.last.as<uint32_t>();
@@ -1045,14 +1082,16 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     hgb[i].tl = m.tl.as<int32_t>();
     hgb[i].ql = m.ql.as<int2>();
     hgb[i].hq = m.hq.as<int2>();
-    hgb[i].ctl = m.ctl.as<Ctl>();
+    hgb[i].ctl = reinterpret_cast<Ctl*>(drun + rb.ctl) + i;
+    hctl[i].ls.n_total = n;  // the device loop reads its run's size here
+    hctl[i].ls.nbatches = rp.nbatches;
     hgb[i].planes = m.planes.as<uint32_t>();
   }
   Params p;
   fill_graph_params(g, o, rp.words, rp.threads, &p);
   if (!devloop) p.sparse_div = 0;
-  p.src = g->d_src.as<int32_t>();
-  p.out_row = g->d_outrow.as<int32_t>();
+  p.src = dsrc;
+  p.out_row = drow;
   p.n_total = n;
   p.C = rp.C;
   p.nbatches = rp.nbatches;
@@ -1060,8 +1099,8 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   p.cpg = rp.cpg;
   p.db = db;
   p.layout = layout;
-  p.groups = g->d_groups.as<GroupBufs>();
-  p.brec = g->d_brec.as<BatchRec>();
+  p.groups = reinterpret_cast<GroupBufs*>(drun + rb.groups);
+  p.brec = reinterpret_cast<BatchRec*>(drun + rb.brec);
   p.lrec = g->d_lrec.as<LevelRec>();
   p.lrec_cap = kLrecCap;
   set_output_params(g, rp.C, dout, &p);
@@ -1082,14 +1121,13 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   p.done_flags = g->d_done;
   // The depth sink: a finished batch's rows (or its vertex-major block) go
   // from `dout` to the caller's host buffer at the same byte offsets.
-  const int32_t* rows_host = g->h_outrow.as<int32_t>();
   auto push_batch = [&](int b) -> cudaError_t {
     const int64_t n_b = std::min<int64_t>(rp.C, n - (int64_t)b * rp.C);
     const size_t rowb = (size_t)g->V * db;
     if (layout == IBFS_LAYOUT_VERTEX_MAJOR)
       return g->sink.push((size_t)b * rowb * rp.C, rowb * (size_t)n_b);
     for (int64_t j = 0; j < n_b; j++) {
-      const cudaError_t e = g->sink.push((size_t)rows_host[(int64_t)b * rp.C + j] * rowb, rowb);
+      const cudaError_t e = g->sink.push((size_t)hrow[(int64_t)b * rp.C + j] * rowb, rowb);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1100,8 +1138,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   std::string key;
   bool replay = false;
   if (use_graph) {
-    const void* extra[] = {g->h_src.p,  g->h_outrow.p, g->h_par.p,  g->d_src.p,
-                           g->d_outrow.p, g->d_groups.p, g->d_brec.p, g->d_lrec.p,
+    const void* extra[] = {g->h_run.p, g->d_run.p, g->d_lrec.p,
                            g->d_out.p,  g->gbin.p,     g->gbkeys.p, g->gbhub.p};
     key = make_key(g, src, n, o, depth_out, layout, flags, rp, p, hgb, rp.G, extra,
                    (int)(sizeof(extra) / sizeof(extra[0])));
@@ -1110,12 +1147,9 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
 
   auto enqueue = [&](cudaStream_t cs, bool capturing) -> ibfs_status {
     {
-      const ibfs_status us = upload_sources(cs);
+      const ibfs_status us = upload(cs);
       if (us != IBFS_OK) return us;
     }
-    CU(cudaMemcpyAsync(g->d_groups.p, hgb, sizeof(GroupBufs) * rp.G, cudaMemcpyHostToDevice, cs));
-    for (int i = 0; i < rp.G; i++) CU(cudaMemsetAsync(hgb[i].ctl, 0, sizeof(Ctl), cs));
-    CU(cudaMemsetAsync(g->d_brec.p, 0, sizeof(BatchRec) * rp.nbatches, cs));
     // inside a capture a plain cudaEventRecord only orders work; an external
     // record becomes a real event-record node that replays time
     if (capturing) CU(cudaEventRecordWithFlags(g->ev0, cs, cudaEventRecordExternal));
@@ -1139,7 +1173,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     if (capturing) CU(cudaEventRecordWithFlags(g->ev1, cs, cudaEventRecordExternal));
     else CU(cudaEventRecord(g->ev1, cs));
     if (rp.host_out) CU(cudaMemcpyAsync(depth_out, dout, out_bytes, cudaMemcpyDeviceToHost, cs));
-    return IBFS_OK;
+    return download(cs);
   };
 
   if (persistent) {
@@ -1181,18 +1215,9 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   } else if (devloop) {
     // ---- device-driven schedule: one graph launch runs every level ------
     {
-      const ibfs_status us = upload_sources(s);
+      const ibfs_status us = upload(s);
       if (us != IBFS_OK) return us;
     }
-    CU(cudaMemcpyAsync(g->d_groups.p, hgb, sizeof(GroupBufs) * rp.G, cudaMemcpyHostToDevice, s));
-    Ctl* hctl = g->h_par.as<Ctl>();  // host staging of the G control blocks
-    for (int i = 0; i < rp.G; i++) {
-      std::memset(&hctl[i], 0, sizeof(Ctl));
-      hctl[i].ls.n_total = n;
-      hctl[i].ls.nbatches = rp.nbatches;
-      CU(cudaMemcpyAsync(hgb[i].ctl, &hctl[i], sizeof(Ctl), cudaMemcpyHostToDevice, s));
-    }
-    CU(cudaMemsetAsync(g->d_brec.p, 0, sizeof(BatchRec) * rp.nbatches, s));
     // the graph bakes in the launch Params (device pointers, graph sizes,
     // options), the group count and the launch shapes: rebuild when any of
     // them moves.  The run's source and batch counts travel in the control
@@ -1229,14 +1254,17 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     }
     if (rp.host_out && dev_gb) {
       // the device GroupBy chose the rows: the sink needs them on the host
-      CU(cudaMemcpyAsync(g->h_outrow.p, g->d_outrow.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost,
-                         s));
+      CU(cudaMemcpyAsync(hrow, drow, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s));
       CU(cudaEventRecord(g->ev_out, s));
     }
     std::memset(g->h_done, 0, sizeof(int32_t) * (size_t)rp.nbatches);
     CU(cudaEventRecord(g->ev0, s));
     CU(cudaGraphLaunch(slot->exec, s));
     CU(cudaEventRecord(g->ev1, s));
+    {
+      const ibfs_status ds = download(s);
+      if (ds != IBFS_OK) return ds;
+    }
     if (rp.host_out) {
       // Stream every batch out as soon as its done flag is up, while the
       // graph keeps traversing the others; batches whose flag never comes
@@ -1268,24 +1296,21 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   } else {
     // ---- plain schedule -------------------------------------------------
     {
-      const ibfs_status us = upload_sources(s);
+      const ibfs_status us = upload(s);
       if (us != IBFS_OK) return us;
     }
-    CU(cudaMemcpyAsync(g->d_groups.p, hgb, sizeof(GroupBufs) * 1, cudaMemcpyHostToDevice, s));
-    CU(cudaMemsetAsync(g->d_brec.p, 0, sizeof(BatchRec) * rp.nbatches, s));
     CU(cudaEventRecord(g->ev0, s));
     const GroupBufs gb = hgb[0];
     const int grid = g->sms, thr = rp.threads;  // launch helpers size each grid
     Par* hpar = reinterpret_cast<Par*>(g->h_par.p);
-    BatchRec* hbr = g->h_brec.as<BatchRec>();
+    BatchRec* hbr = hbrec;
     LevelRec* hlr = g->h_lrec.as<LevelRec>();
     const size_t vpad = (size_t)((g->V + 31) & ~31LL);
     const size_t nchg = (size_t)(((g->V + 31) / 32 + 127) & ~127LL);
     if (rp.host_out) {
       CU(g->sink.begin(g->device, depth_out, dout));
       if (dev_gb) {
-        CU(cudaMemcpyAsync(g->h_outrow.p, g->d_outrow.p, sizeof(int32_t) * n,
-                           cudaMemcpyDeviceToHost, s));
+        CU(cudaMemcpyAsync(hrow, drow, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
       }
     }
@@ -1354,27 +1379,20 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     CU(cudaEventRecord(g->ev1, s));
     if (rp.host_out) CU(g->sink.finish());
   }
-  CU(cudaStreamSynchronize(s));
-  // collect results
-  if (persistent || devloop) {
-    CU(cudaMemcpyAsync(g->h_brec.p, g->d_brec.p, sizeof(BatchRec) * rp.nbatches,
+  if ((persistent || devloop) && st && st->levels && st->levels_cap > 0)
+    CU(cudaMemcpyAsync(g->h_lrec.p, g->d_lrec.p, sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap,
                        cudaMemcpyDeviceToHost, s));
-    if (st && st->levels && st->levels_cap > 0)
-      CU(cudaMemcpyAsync(g->h_lrec.p, g->d_lrec.p, sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap,
-                         cudaMemcpyDeviceToHost, s));
-    int* herr = reinterpret_cast<int*>(g->h_par.p);  // the staged control blocks are done with
-    for (int i = 0; i < rp.G; i++)
-      CU(cudaMemcpyAsync(&herr[i], &hgb[i].ctl->err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
+  CU(cudaStreamSynchronize(s));
+  if (persistent || devloop) {
     int gerr = 0;
     for (int i = 0; i < rp.G; i++)
-      if (herr[i] && !gerr) gerr = herr[i];
+      if (hctl[i].err && !gerr) gerr = hctl[i].err;
     if (gerr) {
       *range_hit = gerr == 3;
       return (ibfs_status)gerr;
     }
   }
-  const BatchRec* br = g->h_brec.as<BatchRec>();
+  const BatchRec* br = hbrec;
   if (st) {
     float ms = -1.0f;
     if (cudaEventElapsedTime(&ms, g->ev0, g->ev1) != cudaSuccess) {

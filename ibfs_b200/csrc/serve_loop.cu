@@ -128,7 +128,7 @@ ibfs_status ServeLoop::init(ibfs_graph* g, const ibfs_opts& o, int G, int slots,
     b.chg = static_cast<uint32_t*>(dalloc(2 * nchg * 4));
     b.planes = static_cast<uint32_t*>(dalloc((size_t)(db == 1 ? 8 : 16) * vpad * words_ * 4));
     b.q = static_cast<int32_t*>(dalloc((size_t)V * 4));
-    b.tl = static_cast<int32_t*>(dalloc((size_t)V * 4));
+    b.tl = static_cast<int32_t*>(dalloc((size_t)std::max<int64_t>(V, kMaxWords * 32) * 4));
     b.ql = static_cast<int2*>(dalloc(capl * 8));
     b.hq = static_cast<int2*>(dalloc((size_t)graph_defer_cap(g) * 8));
     b.ctl = static_cast<Ctl*>(dalloc(sizeof(Ctl)));

@@ -57,7 +57,7 @@ typedef enum ibfs_mode {
        CUDA graph whose conditional nodes run the batch and level loops on
        the device: no host round trip per level, no grid barrier */
     IBFS_MODE_DEVICE_LOOP = 2,
-    /* the default: PERSISTENT (with use_graph) when one batch's status words
+    /* the default: PERSISTENT when one batch's status words
        fit in 32 MB, where per-kernel launch costs would dominate; DEVICE_LOOP
        above that */
     IBFS_MODE_AUTO = 3
