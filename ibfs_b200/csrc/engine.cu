@@ -1145,6 +1145,12 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     replay = g->gcache.exec && g->gcache.key == key;
   }
 
+  // Depths of a persistent run to host memory: from 1 MB on through the sink
+  // (direct when pinned, its staging ring when pageable).  R-MAT scale 12 to
+  // a reused pageable array, one driver copy / ring: 0.5 MB 213 / 214 us,
+  // 1 MB 260 / 217 us, 2 MB 326 / 243 us, 8 MB 715 / 471 us per call.
+  const bool staged = persistent && rp.host_out && !use_graph && out_bytes >= (1u << 20);
+
   auto enqueue = [&](cudaStream_t cs, bool capturing) -> ibfs_status {
     {
       const ibfs_status us = upload(cs);
@@ -1172,7 +1178,8 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     }
     if (capturing) CU(cudaEventRecordWithFlags(g->ev1, cs, cudaEventRecordExternal));
     else CU(cudaEventRecord(g->ev1, cs));
-    if (rp.host_out) CU(cudaMemcpyAsync(depth_out, dout, out_bytes, cudaMemcpyDeviceToHost, cs));
+    if (rp.host_out && !staged)
+      CU(cudaMemcpyAsync(depth_out, dout, out_bytes, cudaMemcpyDeviceToHost, cs));
     return download(cs);
   };
 
@@ -1211,6 +1218,12 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     } else {
       ibfs_status es2 = enqueue(s, false);
       if (es2 != IBFS_OK) return es2;
+      if (staged) {
+        CU(g->sink.begin(g->device, depth_out, dout));
+        CU(g->sink.wait_for(g->ev1));
+        CU(g->sink.push(0, out_bytes));
+        CU(g->sink.finish());
+      }
     }
   } else if (devloop) {
     // ---- device-driven schedule: one graph launch runs every level ------

@@ -172,8 +172,8 @@ class DepthSink {
   bool pinned() const { return pinned_; }
 
  private:
-  static constexpr int kSlots = 4;
-  static constexpr size_t kSlotBytes = 32u << 20;
+  static constexpr int kSlots = 8;
+  static constexpr size_t kSlotBytes = 4u << 20;
   struct Piece {
     size_t off, at, bytes;  // output offset, offset in the slot, length
   };
