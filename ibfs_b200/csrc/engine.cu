@@ -196,8 +196,8 @@ struct ibfs_graph {
   DevBuf beg, col;
   DevBuf gbhub;         // GroupBy's hub of every vertex (-1: not eligible), device GroupBy
   DevBuf vmap;          // caller id -> internal id (device)
-  std::vector<int32_t> new_of_old;  // the same on the host
-  std::vector<int64_t> dbeg_host;   // offsets of the internal (degree-ordered) CSR
+  HostArray<int32_t> new_of_old;    // the same on the host
+  HostArray<int64_t> dbeg_host;     // offsets of the internal (degree-ordered) CSR
   int64_t col_max = -1;             // largest neighbour id of the internal CSR
   DevBuf gbin, gbkeys;  // device GroupBy: caller-order sources, sort keys
   int64_t defer_cap = 16;  // bound on deferred bottom-up hub chunks per level
@@ -546,38 +546,14 @@ extern "C" void ibfs_opts_default(ibfs_opts* o) {
   o->bu_thread_max = 32;
 }
 
-static ibfs_status upload_graph(ibfs_graph* g) {
-  CU(cudaSetDevice(g->device));
-  int sms = 0;
-  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
-  g->sms = sms;
-  ibfs_status s;
-  if ((s = g->beg.ensure(sizeof(int64_t) * (size_t)(g->V + 1))) != IBFS_OK) return s;
-  // + 4 entries: the bottom-up reads column ids as aligned 16-byte vectors
-  if ((s = g->col.ensure(sizeof(int32_t) * (size_t)(g->E + 4))) != IBFS_OK) return s;
-  CU(cudaMemset(g->col.p, 0, sizeof(int32_t) * (size_t)(g->E + 4)));
-  CU(cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking));
-  g->stream = g->own_stream;
-  CU(cudaEventCreate(&g->ev0));
-  CU(cudaEventCreate(&g->ev1));
-  CU(cudaEventCreateWithFlags(&g->ev_out, cudaEventDisableTiming));
-  // Internal vertex order: by degree, highest first (ties by caller id).
-  // Vertices of similar degree then share warps (the bottom-up thread path
-  // runs lanes of equal trip counts) and the hubs' status words, which most
-  // gathers hit, are packed into a few contiguous lines of L2 -- measured on
-  // R-MAT scale 24: 45.5 -> 27.6 ms per 1024-source run.  Depths do not
-  // depend on the order: sources are renamed on the way in, and the output
-  // pass reads statuses through the map, writing rows in the caller's order.
-  // The device adjacency lists are in this order too, sorted ascending,
-  // which is by neighbour degree, highest first: the bottom-up sweep stops at
-  // the first neighbours that cover the missing bits, and hubs carry the
-  // most bits earliest.  The host copy keeps the caller's order (GroupBy's
-  // "first hub in CSR order" and the byte model use it).
+// The internal order built on the host: small graphs, and graphs whose sort
+// scratch does not fit the GPU.
+static ibfs_status order_on_host(ibfs_graph* g) {
   {
     const int64_t* bg = g->h.beg.data();
     const int32_t* cl = g->h.col.data();
     std::vector<int32_t> order;
-    std::vector<int64_t> nbeg;
+    HostArray<int64_t>& nbeg = g->dbeg_host;
     std::vector<int32_t> dcol;
     try {
       order.resize((size_t)g->V);
@@ -611,12 +587,9 @@ static ibfs_status upload_graph(ibfs_graph* g) {
     g->col_max = col_max;
     CU(cudaMemcpyAsync(g->beg.p, nbeg.data(), sizeof(int64_t) * (size_t)(g->V + 1),
                        cudaMemcpyHostToDevice, g->stream));
-    g->dbeg_host = nbeg;  // (the copy is synchronised below)
     if (g->E)
       CU(cudaMemcpyAsync(g->col.p, dcol.data(), sizeof(int32_t) * (size_t)g->E,
                          cudaMemcpyHostToDevice, g->stream));
-    if ((s = g->vmap.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(g->V, 1))) != IBFS_OK)
-      return s;
     CU(cudaMemcpyAsync(g->vmap.p, nmap, sizeof(int32_t) * (size_t)g->V, cudaMemcpyHostToDevice,
                        g->stream));
     CU(cudaStreamSynchronize(g->stream));
@@ -645,26 +618,85 @@ static ibfs_status upload_graph(ibfs_graph* g) {
         }
       }
     }
-    if ((s = g->gbhub.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(g->V, 1))) != IBFS_OK)
-      return s;
     CU(cudaMemcpyAsync(g->gbhub.p, hub.data(), sizeof(int32_t) * (size_t)g->V,
                        cudaMemcpyHostToDevice, g->stream));
     CU(cudaStreamSynchronize(g->stream));
   }
-  CU(cudaStreamSynchronize(g->stream));
-  int64_t md = 0;
-  for (int64_t v = 0; v < g->V; v++) md = std::max(md, g->h.beg[v + 1] - g->h.beg[v]);
-  g->max_deg = md;
-  // bound on the bottom-up hub chunks one level can defer
-  {
-    int64_t cap = 16;
-    for (int64_t v = 0; v < g->V; v++) {
-      const int64_t d = g->h.beg[v + 1] - g->h.beg[v];
-      if (d > kHubScan) cap += (d - kHubScan + kHubChunk - 1) / kHubChunk;
-    }
-    g->defer_cap = cap;
-  }
   return IBFS_OK;
+}
+
+// Below this many edges the host's sort is done before the GPU's kernels are
+// launched.  ibfs_graph_from_csr on the host / on the GPU, best of 12: R-MAT
+// scale 10 (12 k edges) 0.97 / 0.82 ms, scale 11 (46 k) 1.62 / 1.21 ms, scale
+// 14 (0.43 M) 11.5 / 1.6 ms, scale 18 (7.6 M) 176 / 6.1 ms, scale 22 (128 M)
+// 1,987 / 110 ms.
+static const int64_t kHostOrderEdges = 1 << 13;
+
+static ibfs_status upload_graph(ibfs_graph* g) {
+  CU(cudaSetDevice(g->device));
+  int sms = 0;
+  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
+  g->sms = sms;
+  ibfs_status s;
+  if ((s = g->beg.ensure(sizeof(int64_t) * (size_t)(g->V + 1))) != IBFS_OK) return s;
+  // + 4 entries: the bottom-up reads column ids as aligned 16-byte vectors
+  if ((s = g->col.ensure(sizeof(int32_t) * (size_t)(g->E + 4))) != IBFS_OK) return s;
+  CU(cudaMemset(g->col.p, 0, sizeof(int32_t) * (size_t)(g->E + 4)));
+  CU(cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking));
+  g->stream = g->own_stream;
+  CU(cudaEventCreate(&g->ev0));
+  CU(cudaEventCreate(&g->ev1));
+  CU(cudaEventCreateWithFlags(&g->ev_out, cudaEventDisableTiming));
+  if ((s = g->vmap.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(g->V, 1))) != IBFS_OK)
+    return s;
+  if ((s = g->gbhub.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(g->V, 1))) != IBFS_OK)
+    return s;
+  // the largest degree, and a bound on the bottom-up hub chunks one level can
+  // defer
+  const int64_t* bg = g->h.beg.data();
+  int64_t md = 0, cap = 16;
+#pragma omp parallel for schedule(static) reduction(max : md) reduction(+ : cap)
+  for (int64_t v = 0; v < g->V; v++) {
+    const int64_t d = bg[v + 1] - bg[v];
+    md = std::max(md, d);
+    if (d > kHubScan) cap += (d - kHubScan + kHubChunk - 1) / kHubChunk;
+  }
+  g->max_deg = md;
+  g->defer_cap = cap;
+  // Internal vertex order: by degree, highest first (ties by caller id).
+  // Vertices of similar degree then share warps (the bottom-up thread path
+  // runs lanes of equal trip counts) and the hubs' status words, which most
+  // gathers hit, are packed into a few contiguous lines of L2 -- measured on
+  // R-MAT scale 24: 45.5 -> 27.6 ms per 1024-source run.  Depths do not
+  // depend on the order: sources are renamed on the way in, and the output
+  // pass reads statuses through the map, writing rows in the caller's order.
+  // The device adjacency lists are in this order too, sorted ascending,
+  // which is by neighbour degree, highest first: the bottom-up sweep stops at
+  // the first neighbours that cover the missing bits, and hubs carry the
+  // most bits earliest.  The host copy keeps the caller's order (GroupBy's
+  // "first hub in CSR order" and the byte model use it).
+  if (g->E >= kHostOrderEdges && g->E < INT32_MAX) {
+    const cudaError_t pe =
+        prep_graph(bg, g->h.col.data(), g->V, g->E, md, g->beg.as<int64_t>(),
+                   g->col.as<int32_t>(), g->vmap.as<int32_t>(), g->gbhub.as<int32_t>(),
+                   &g->col_max, g->stream);
+    if (pe == cudaSuccess) {
+      try {
+        g->new_of_old.resize((size_t)g->V);
+        g->dbeg_host.resize((size_t)g->V + 1);
+      } catch (const std::bad_alloc&) {
+        return IBFS_ERR_OOM;
+      }
+      CU(cudaMemcpyAsync(g->new_of_old.data(), g->vmap.p, sizeof(int32_t) * (size_t)g->V,
+                         cudaMemcpyDeviceToHost, g->stream));
+      CU(cudaMemcpyAsync(g->dbeg_host.data(), g->beg.p, sizeof(int64_t) * (size_t)(g->V + 1),
+                         cudaMemcpyDeviceToHost, g->stream));
+      CU(cudaStreamSynchronize(g->stream));
+      return IBFS_OK;
+    }
+    if (pe != cudaErrorMemoryAllocation) CU(pe);
+  }
+  return order_on_host(g);
 }
 
 static void destroy_graph(ibfs_graph* g) {
@@ -728,8 +760,8 @@ extern "C" ibfs_status ibfs_graph_from_csr(const int64_t* beg_pos_host, const in
   try {
     g->h.V = V;
     g->h.E = E;
-    g->h.beg.assign(beg_pos_host, beg_pos_host + V + 1);
-    g->h.col.assign(col_host, col_host + E);
+    g->h.beg.copy_from(beg_pos_host, (size_t)(V + 1));
+    g->h.col.copy_from(col_host, (size_t)E);
   } catch (const std::bad_alloc&) {
     delete g;
     return IBFS_ERR_OOM;

@@ -61,7 +61,8 @@ ibfs_status build_csr(const int32_t* u, const int32_t* v, int64_t m, int64_t V,
       deg[x] = std::unique(s, e) - s;
     }
     out->V = V;
-    out->beg.assign(V + 1, 0);
+    out->beg.resize((size_t)(V + 1));
+    out->beg[0] = 0;
     for (int64_t i = 0; i < V; i++) out->beg[i + 1] = out->beg[i] + deg[i];
     out->E = out->beg[V];
     out->col.resize((size_t)out->E);

@@ -3,6 +3,9 @@
 #include <cstdint>
 #include <algorithm>
 #include <cstddef>
+#include <cstdlib>
+#include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -26,11 +29,55 @@ static inline uint64_t rnd(uint64_t seed, uint64_t stream, uint64_t i) {
 }
 
 // Host CSR (int64 offsets, int32 column ids).
+// An array of the host CSR's size: not zeroed when it is sized (its pages are
+// first touched by whoever fills it, all cores at once), freed on destruction.
+// Throws std::bad_alloc like a vector.
+template <class T>
+class HostArray {
+ public:
+  HostArray() = default;
+  HostArray(const HostArray&) = delete;
+  HostArray& operator=(const HostArray&) = delete;
+  ~HostArray() { std::free(p_); }
+  void resize(size_t n) {
+    std::free(p_);
+    n_ = 0;
+    p_ = static_cast<T*>(std::malloc(std::max<size_t>(n, 1) * sizeof(T)));
+    if (!p_) throw std::bad_alloc();
+    n_ = n;
+  }
+  void copy_from(const T* src, size_t n) {
+    resize(n);
+    constexpr size_t kPiece = (256u << 10) / sizeof(T);
+    const long long cuts = (long long)((n + kPiece - 1) / kPiece);
+#pragma omp parallel for schedule(static) if (cuts > 2)
+    for (long long i = 0; i < cuts; i++) {
+      const size_t at = (size_t)i * kPiece;
+      std::memcpy(p_ + at, src + at, std::min(kPiece, n - at) * sizeof(T));
+    }
+  }
+  T* data() { return p_; }
+  const T* data() const { return p_; }
+  size_t size() const { return n_; }
+  T& operator[](size_t i) { return p_[i]; }
+  const T& operator[](size_t i) const { return p_[i]; }
+
+ private:
+  T* p_ = nullptr;
+  size_t n_ = 0;
+};
+
 struct HostCsr {
   int64_t V = 0, E = 0;
-  std::vector<int64_t> beg;
-  std::vector<int32_t> col;
+  HostArray<int64_t> beg;
+  HostArray<int32_t> col;
 };
+
+// prep.cu: the internal vertex order, the renamed and sorted adjacency lists
+// and GroupBy's hub table, built on the GPU.
+cudaError_t prep_graph(const int64_t* beg_h, const int32_t* col_h, int64_t V, int64_t E,
+                       int64_t max_deg, int64_t* beg, int32_t* col, int32_t* vmap, int32_t* hub,
+                       int64_t* col_max, cudaStream_t s);
 
 // Symmetrise, drop self-loops, sort and dedupe every adjacency list.
 ibfs_status build_csr(const int32_t* u, const int32_t* v, int64_t m, int64_t V,
