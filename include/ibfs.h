@@ -79,7 +79,8 @@ typedef enum ibfs_layout {
 typedef struct ibfs_graph ibfs_graph;
 
 typedef struct ibfs_opts {
-    int32_t width;         /* status bits per vertex: 32, 64, 128 or 256          */
+    int32_t width;         /* status bits per vertex: 32, 64, 128 or 256 (fewer are
+                              kept when a batch has fewer sources)            */
     int32_t concurrent;    /* sources per batch, 1..width (0: width)              */
     int32_t switch_level;  /* >= 0: fixed switch as the reference's CLI argument:
                               top-down while level <= switch_level, bottom-up after;
@@ -148,7 +149,8 @@ typedef struct ibfs_stats {
     int64_t n_batches;
     int32_t max_level;      /* deepest BFS level over all sources                 */
     int32_t depth_bytes;    /* depth type actually used                           */
-    int32_t width;          /* status width actually used                         */
+    int32_t width;          /* status width of the options (a run keeps only the
+                               words its largest batch needs)                     */
     int32_t groups;         /* concurrent batches per launch actually used        */
     int64_t levels_total;   /* sum over batches of levels expanded                */
     int64_t td_levels;
