@@ -235,7 +235,7 @@ static const int kLrecCap = 1024;
 // many as those need, at most the width asked for.  Bits that no source owns
 // would be read and written with every status all the same: one source on the
 // 3.07 M vertex social graph (width 128) takes 513 us in four words, 390 us
-// in one; a 1800 x 1800 grid, 1 source, 21.2 ms with 128 sources' words, 3.2 ms.
+// in one.
 static int words_used(int width, int64_t n_b) {
   int w = 1;
   while (w < width / 32 && w * 32 < n_b) w *= 2;
@@ -479,7 +479,6 @@ void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int t
 // The output pointer and the store widths its alignment allows.
 void set_output_params(const ibfs_graph* g, int C, uint8_t* dout, Params* p) {
   p->out = dout;
-  p->vec_out = (C % 4 == 0) && ((reinterpret_cast<uintptr_t>(dout) & 3) == 0);
   p->vec_sm = (g->V % 16 == 0 && (reinterpret_cast<uintptr_t>(dout) & 15) == 0)  ? 16
               : (g->V % 4 == 0 && (reinterpret_cast<uintptr_t>(dout) & 3) == 0) ? 4
                                                                                : 0;

@@ -165,7 +165,6 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   p.brec = reinterpret_cast<BatchRec*>(base + o_brec);
   p.lrec = nullptr;  // no level records
   p.lrec_cap = 0;
-  p.vec_out = ((reinterpret_cast<uintptr_t>(depth_dev) & 3) == 0) ? 1 : 0;
   p.hub_t = INT32_MAX;  // no deferred hub chunks here: the sweep scans whole lists
   p.bu_filter = 0;
   p.col_vec = 0;  // the caller's col is neither known to be padded nor aligned
