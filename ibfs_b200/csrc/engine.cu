@@ -1007,10 +1007,18 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   if (persistent) {
     int G = o.groups;
     if (G == 0) {
-      // enough CTAs per group to sweep V with >= 8 words of 32 vertices per warp
-      const int64_t want = std::max<int64_t>(1, (g->V + 32LL * 8 * (rp.threads / 32) - 1) /
-                                                    (32LL * 8 * (rp.threads / 32)));
+      // A group's CTAs sweep at least `share` vertices each; below that more
+      // groups only multiply the batches in flight.  Among the counts that
+      // leave, the largest that shares the batches out evenly (to 15 %): a
+      // last batch that runs alone has one group's share of the GPU.
+      // Measured, 1 / 2 / 3 / 4 / 8 groups: R-MAT scale 18, 8 batches of 128
+      // 2644 / 1617 / 1703 / 1397 / 1531 us; 500,009 vertices, 3 batches of
+      // 250 2184 / 2405 / 1772 us; scale 20, 2 batches of 32 864 / 792 us, of
+      // 128 (wider words, more of L2 per batch) 1829 / 1986 us.
+      const int64_t share = rp.words <= 2 ? 8192 : 6144;
+      const int64_t want = std::max<int64_t>(1, g->V * 512 / (share * rp.threads));
       G = (int)std::max<int64_t>(1, std::min<int64_t>(rp.nbatches, total_ctas / std::min<int64_t>(want, total_ctas)));
+      while (G > 1 && (int64_t)((rp.nbatches + G - 1) / G) * G * 100 > (int64_t)rp.nbatches * 115) G--;
       // memory guard (only when the workspace has to grow to G groups)
       size_t freeb = 0, totb = 0;
       if ((int)g->groups.size() < G && cudaMemGetInfo(&freeb, &totb) == cudaSuccess) {

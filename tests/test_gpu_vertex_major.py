@@ -14,7 +14,8 @@ _CACHE = {}
 
 def graph(V):
     if V not in _CACHE:
-        beg, col = ib.gen_chung_lu(V, 4 * V, 2.1, V / 4, seed=V)
+        u, v = np.random.default_rng(V).integers(0, V, (2, 3 * V)).astype(np.int32)
+        beg, col = ib.csr_from_edges(u, v, V)
         _CACHE[V] = (beg, col, ib.Graph.from_csr(beg, col))
     return _CACHE[V]
 
