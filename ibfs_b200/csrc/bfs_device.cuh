@@ -84,6 +84,7 @@ struct __align__(256) Ctl {
   int err;
   int pad0[2];
   Par par[3];
+  int32_t tail_src;  // a source of the batch lies at or past Params::v_reach
   __align__(16) int32_t qc[2][4];  // [consumer level parity][small, medium, large-chunks]
   unsigned long long pad1[4];
   LoopState ls;
@@ -519,6 +520,7 @@ __device__ void seed_phase(const Params& p, const GroupBufs& gb,
   for (long long i = t.tid; i < n_b; i += t.nthreads) {
     const int32_t v = src_b[i];
     atomicOr(gb.curr + (size_t)v * WORDS + (i >> 5), 1u << (i & 31));
+    if (v >= p.v_reach) gb.ctl->tail_src = 1;
     const uint32_t bit = 1u << (v & 31);
     const uint32_t old = atomicOr(chg0 + (v >> 5), bit);
     if (THIN && !(old & bit)) gb.tl[atomicAdd(&gb.ctl->par[0].t_cnt, 1)] = v;
@@ -2045,6 +2047,7 @@ __device__ void output_sm_u8(const Params& p, const GroupBufs& gb, const int32_t
                              const Team& t) {
   static_assert(NP <= 8, "one-byte depths use at most 8 planes");
   const int lane = t.lane;
+  const bool tail_src = gb.ctl->tail_src != 0;
   for (long long base = t.warp * 128; base < p.V; base += t.nwarps * 128) {
     const long long v0 = base + 4 * lane;
     const bool full4 = p.vec_sm >= 4 && v0 + 3 < p.V;
@@ -2055,6 +2058,7 @@ __device__ void output_sm_u8(const Params& p, const GroupBufs& gb, const int32_t
       vis[i] = v0 + i < p.V ? (uint32_t)(p.vmap ? p.vmap[v0 + i] : v0 + i) : 0u;
 #pragma unroll 1
     for (int k = 0; k < WORDS && k * 32 < n_b; k++) {
+      const uint32_t mine = full_word(n_b, k);
       uint32_t A[32];
 #pragma unroll
       for (int i = 0; i < 4; i++) {
@@ -2064,23 +2068,26 @@ __device__ void output_sm_u8(const Params& p, const GroupBufs& gb, const int32_t
         // its plane words are zeros (every plane was first written whole
         // during the batch), so they are not gathered
         const bool edged = in && (long long)vi < p.v_reach;
-        const uint32_t nst = in ? ~gb.last[vi * WORDS + k] : 0xFFFFFFFFu;
+        uint32_t some = 0u;  // sources with a plane bit: reached, depth > 0
+#pragma unroll
+        for (int b = 0; b < NP; b++) {
+          A[8 * i + b] = edged ? gb.planes[(size_t)b * p.plane_stride + vi * WORDS + k] : 0u;
+          some |= A[8 * i + b];
+        }
+        // the others are unreached or the vertex itself: only their status
+        // tells, so the status word is gathered where there are such sources
+        // (past v_reach: when the batch has a source there)
+        uint32_t nst = ~some;
+        if (in && (edged ? (some & mine) != mine : tail_src)) nst = ~gb.last[vi * WORDS + k];
         if constexpr (NP <= 7) {
           // planes in rows 0..NP-1, zero rows up to 6 (folded away by the
           // compiler), the unreached flag in row 7
 #pragma unroll
-          for (int b = 0; b < 7; b++)
-            A[8 * i + b] = (b < NP && edged)
-                               ? gb.planes[(size_t)b * p.plane_stride + vi * WORDS + k]
-                               : 0u;
+          for (int b = NP; b < 7; b++) A[8 * i + b] = 0u;
           A[8 * i + 7] = nst;
         } else {
 #pragma unroll
-          for (int b = 0; b < 8; b++) {
-            uint32_t x = 0u;
-            if (edged) x = gb.planes[(size_t)b * p.plane_stride + vi * WORDS + k];
-            A[8 * i + b] = x | nst;
-          }
+          for (int b = 0; b < 8; b++) A[8 * i + b] |= nst;
         }
       }
 #if IBFS_OUT_PRMT

@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(512) k_dl_batch_init(Params p, int g, CondH h_
   if (t.warp == 0) {
     for (int i = 0; i < 3; i++) zero_par(&gb.ctl->par[i], t.lane);
     if (t.lane < 8) (&gb.ctl->qc[0][0])[t.lane] = 0;
+    if (t.lane == 8) gb.ctl->tail_src = 0;
   }
   if (t.tid == 0) {
     Ctl* ctl = gb.ctl;

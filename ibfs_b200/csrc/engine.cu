@@ -1013,11 +1013,13 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
       // last batch that runs alone has one group's share of the GPU.
       // Measured, 1 / 2 / 3 / 4 / 8 groups: R-MAT scale 18, 8 batches of 128
       // 2644 / 1617 / 1703 / 1397 / 1531 us; 500,009 vertices, 3 batches of
-      // 250 2184 / 2405 / 1772 us; scale 20, 2 batches of 32 864 / 792 us, of
+      // 250 2184 / 2405 / 1772 us; scale 20, 2 batches of 32 869 / 787 us, of
       // 128 (wider words, more of L2 per batch) 1829 / 1986 us.
       const int64_t share = rp.words <= 2 ? 8192 : 6144;
       const int64_t want = std::max<int64_t>(1, g->V * 512 / (share * rp.threads));
       G = (int)std::max<int64_t>(1, std::min<int64_t>(rp.nbatches, total_ctas / std::min<int64_t>(want, total_ctas)));
+      // a graph that fills the GPU by itself (team_ctas) takes four at most
+      if (g->E / 12288 >= total_ctas) G = std::min(G, 4);
       while (G > 1 && (int64_t)((rp.nbatches + G - 1) / G) * G * 100 > (int64_t)rp.nbatches * 115) G--;
       // memory guard (only when the workspace has to grow to G groups)
       size_t freeb = 0, totb = 0;

@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
     if (t.block == 0 && threadIdx.x < 32) {
       for (int i = 0; i < 3; i++) zero_par(&ctl->par[i], t.lane);
       if (threadIdx.x < 8) (&ctl->qc[0][0])[threadIdx.x] = 0;
+      if (threadIdx.x == 8) ctl->tail_src = 0;
     }
     BARRIER();
     seed_phase<WORDS, true>(p, gb, p.src + k0, n_b, t);
