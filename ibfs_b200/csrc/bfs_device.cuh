@@ -72,7 +72,7 @@ struct LoopState {
                               // (batch_end clears its unreachable sources' words)
   int32_t sparse_try;         // this bottom-up level follows a top-down one: count
                               // the sources' frontiers and pick the sparse ones
-  int32_t thin;               // `level` collects its changed vertices in the touched list
+  int32_t kind;               // how `level` keeps track of its changed vertices (td_kind)
   int32_t have_q;             // the queues of `level` were built by the previous inspect
   unsigned long long m_u, teps, prev_changed;
   unsigned long long t_lvl, t_mid;  // %globaltimer at the level start / inspect start
@@ -227,6 +227,33 @@ template <bool RO>
 __device__ __forceinline__ bool in_front(const uint32_t* front, int32_t u) {
   const uint32_t w = RO ? __ldg(front + (u >> 5)) : __ldcg(front + (u >> 5));
   return (w >> (u & 31)) & 1u;
+}
+
+// How a top-down level keeps track of the vertices it changes.
+//   thin   a list: the first push to change a vertex appends it (one returned
+//          atomic), and the inspect step, which reads only the list, queues the
+//          next level on the way;
+//   bitmap every push that adds bits marks its vertex;
+//   wide   nothing: the inspect step compares every vertex's two statuses, in
+//          one coalesced sweep, and writes the bitmap itself.
+// What a level costs beside its pushes: one appended counter (thin), one more
+// reduction per push (bitmap), a sweep of 32 to 64 bytes per reachable vertex
+// (wide).  So a frontier of at most 2^20 edges is thin -- with the limit at
+// 2^17 / 2^20 / 2^23 edges R-MAT scale 22, 512 sources takes 5.10 / 5.06 / 5.14
+// ms, a grid of 4096^2, 256 sources 156.1 / 154.1 / 157.9 ms, R-MAT scale
+// 20, 60 sources in 32-bit words 1.55 / 1.56 / 1.61 ms -- and one with an edge
+// per two reachable vertices is wide -- at 1/4 / 1 / 4 edges per vertex
+// scale 22 takes 4.40 / 4.48 / 4.65 ms, the grid 153.7 / 152.9 / 152.8 ms,
+// scale 20 0.79 / 0.79 / 0.84 ms.  The pushes are bound by L2's reductions:
+// without the bitmap's the level that pushes 30 M edges of the social graph
+// went from 609 to 354 us, its inspect step from 100 to 61 us (coalesced).
+constexpr int kTdBitmap = 0;
+constexpr int kTdThin = 1;
+constexpr int kTdWide = 2;
+constexpr unsigned long long kThinEdges = 1ull << 20;
+__host__ __device__ inline int td_kind(unsigned long long mf, long long v_reach) {
+  if (mf <= kThinEdges) return kTdThin;
+  return mf * 2 >= (unsigned long long)v_reach ? kTdWide : kTdBitmap;
 }
 
 constexpr int kHubScan = 1024;   // neighbours one warp scans before deferring
@@ -544,10 +571,10 @@ __device__ __forceinline__ void inspect_vertex(const Params& p, const GroupBufs&
                                                const uint32_t (&full)[WORDS], uint32_t (&fm)[WORDS],
                                                unsigned long long& mf, unsigned long long& cnt,
                                                unsigned long long& cdeg,
-                                               unsigned long long& teps, long long& deg) {
-  uint32_t c[WORDS], l[WORDS], nb[WORDS];
-  ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
-  ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
+                                               unsigned long long& teps, long long& deg,
+                                               const uint32_t (&c)[WORDS],
+                                               const uint32_t (&l)[WORDS]) {
+  uint32_t nb[WORDS];
   bool comp = true;
   uint32_t pop = 0;
 #pragma unroll
@@ -691,12 +718,8 @@ __device__ __forceinline__ void q_append(const Params& p, const GroupBufs& gb, i
 
 // ---------------------------------------------------------------------------
 // Phase: inspect level L.  Fixes last, updates the depth bit-planes and the
-// counters of every changed vertex.
-//   thin levels (kThinEdges) read the level's touched list and queue the
-//     vertices for the next top-down level on the way, so such a level reads
-//     nothing in proportion to the graph and needs no queue build;
-//   the others walk the level's bitmap.
-// What bounds a thin level is its chain of dependent L2 reads (queue entry,
+// counters of every changed vertex, which it takes
+// vertices from the list, the bitmap or a sweep (td_kind).  What bounds a thin level is its chain of dependent L2 reads (queue entry,
 // offsets, column id, status, then list entry, statuses, planes), so the
 // step is one vertex per lane and 8 lanes per pushed small vertex.  A
 // 256 x 1024 grid without shortcuts (64 sources, 1269 levels, about 12,500
@@ -705,7 +728,7 @@ __device__ __forceinline__ void q_append(const Params& p, const GroupBufs& gb, i
 // ---------------------------------------------------------------------------
 template <int WORDS>
 __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, int n_b,
-                              int level, bool depth_ok, bool thin, int32_t* qc_next,
+                              int level, bool depth_ok, int kind, int32_t* qc_next,
                               const Team& t) {
   uint32_t full[WORDS];
 #pragma unroll
@@ -718,39 +741,56 @@ __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, in
   // bottom-up merges into it with atomics
   zero_words(chg_at(gb, p, level + 1), p.chg_stride, t);
   const int lane = t.lane;
-  if (thin) {
+  if (kind == kTdThin) {
     const int n = __ldcg(&par->t_cnt);
     for (long long base = t.warp * 32; base < n; base += t.nwarps * 32) {
       int32_t v = -1;
       long long deg = 0;
       if (base + lane < n) {
         v = __ldcg(gb.tl + base + lane);
-        inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg);
+        uint32_t c[WORDS], l[WORDS];
+        ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
+        ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
+        inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg, c, l);
       }
       q_append(p, gb, qc_next, lane, v, deg, deg_class(p, deg));
+    }
+  } else if (kind == kTdWide) {
+    uint32_t* chg = chg_at(gb, p, level);
+    for (long long base = t.warp * 32; base < p.v_reach; base += t.nwarps * 32) {
+      const long long v = base + lane;
+      bool ch = false;
+      if (v < p.V) {
+        uint32_t c[WORDS], l[WORDS];
+        ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
+        ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
+#pragma unroll
+        for (int k = 0; k < WORDS; k++) ch |= c[k] != l[k];
+        long long deg;
+        if (ch)
+          inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg, c,
+                                l);
+      }
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, ch);
+      if (lane == 0 && bal) __stcg(chg + (base >> 5), bal);
     }
   } else {
     walk_changed(chg_at(gb, p, level), p.nchg, t,
                  [&](long long v0, const uint16_t* ids, int total) {
                    for (int r = lane; r < total; r += 32) {
+                     const long long v = v0 + ids[r];
                      long long deg;
-                     inspect_vertex<WORDS>(p, gb, v0 + ids[r], level, depth_ok, full, fm, mf, cnt,
-                                           cdeg, teps, deg);
+                     uint32_t c[WORDS], l[WORDS];
+                     ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
+                     ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
+                     inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg,
+                                           teps, deg, c, l);
                    }
                  });
   }
   if (!depth_ok && cnt) par->range_err = 1;
   cta_flush<WORDS>(par, cnt, mf, cdeg, teps, fm);
 }
-
-// A top-down level is thin when the frontier it pushes has at most this many
-// edges: its changed vertices then go through the touched list (one returned
-// atomic per first touch, one list append per warp step).  Above it the
-// appends to one counter cost more than a walk of the bitmap.  Measured with
-// the limit at 2^17 / 2^20 / 2^23 edges: R-MAT scale 22, 512 sources 5.10 /
-// 5.06 / 5.14 ms; grid 4096^2, 256 sources 156.1 / 154.1 / 157.9 ms; R-MAT
-// scale 20, 60 sources in 32-bit words 1.55 / 1.56 / 1.61 ms.
-constexpr unsigned long long kThinEdges = 1ull << 20;
 
 // ---------------------------------------------------------------------------
 // Phase: build the joint frontier queues of top-down level L from the
@@ -844,12 +884,12 @@ __device__ __forceinline__ void red_or_u64(unsigned long long* p, unsigned long 
 // goes on instead of waiting for L2 round trips.  A stale s (fewer bits)
 // costs at most one redundant OR.
 //
-// THIN (the level keeps a touched list): the bitmap OR returns the old word,
+// Thin levels (td_kind): the bitmap OR returns the old word,
 // which says whether this push was the first to change u at this level, and
 // the warp appends those vertices to the list with one atomic per step.  All
 // 32 lanes call it together (cnt 0: nothing to push).
 constexpr int kTdStep = 4;  // edges one thread has in flight
-template <int WORDS, bool THIN>
+template <int WORDS, int KIND>
 __device__ __forceinline__ void td_push_n(const GroupBufs& gb, uint32_t* chg, int32_t* t_cnt,
                                           const int32_t (&u)[kTdStep], int cnt,
                                           const uint32_t (&P)[WORDS]) {
@@ -881,13 +921,13 @@ __device__ __forceinline__ void td_push_n(const GroupBufs& gb, uint32_t* chg, in
       }
     }
     const uint32_t bit = 1u << (u[i] & 31);
-    if constexpr (THIN) {
+    if constexpr (KIND == kTdThin) {
       if (!(atomicOr(chg + (u[i] >> 5), bit) & bit)) first |= 1u << i;
-    } else {
+    } else if constexpr (KIND == kTdBitmap) {
       red_or_u32(chg + (u[i] >> 5), bit);
     }
   }
-  if constexpr (THIN) {
+  if constexpr (KIND == kTdThin) {
     if (!__any_sync(0xFFFFFFFFu, first != 0u)) return;
     const int lane = threadIdx.x & 31;
     const int own = __popc(first);
@@ -954,6 +994,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 
 constexpr int kStageInts = 2048 + 8;  // one chunk (threads*4 <= 2048) plus alignment slack
 
+// The two staging buffers (one array for every instance of the phase).
+__device__ __forceinline__ int32_t (*td_stage_buf())[kStageInts] {
+  __shared__ __align__(128) int32_t s_col[2][kStageInts];
+  return s_col;
+}
+
 // The column-id range [a0, a1) that covers chunk c of a large vertex with
 // 16-byte aligned ends (col is 16-byte aligned and padded by 4 entries).
 __device__ __forceinline__ void td_chunk(const Params& p, const GroupBufs& gb, int c, int32_t* v,
@@ -982,7 +1028,7 @@ __device__ __forceinline__ void td_chunk(const Params& p, const GroupBufs& gb, i
 // on R-MAT scale 24 the top-down levels are bound by the random status
 // gathers, not by the column reads, and staging measured ~1 % slower.
 // ---------------------------------------------------------------------------
-template <int WORDS, bool STAGE, bool THIN>
+template <int WORDS, bool STAGE, int KIND>
 __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int level,
                                        const int32_t* qc, const Team& t) {
   uint32_t* chg = chg_at(gb, p, level);
@@ -990,7 +1036,7 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
   const int4 nq = __ldcg(reinterpret_cast<const int4*>(qc));  // small, medium, large chunks
   const int nS = nq.x, nM = nq.y, nL = nq.z;
   if (STAGE && p.td_stage) {
-    __shared__ __align__(128) int32_t s_col[2][kStageInts];
+    int32_t (*s_col)[kStageInts] = td_stage_buf();
     __shared__ __align__(8) unsigned long long s_bar[2];
     __shared__ int s_fail;
     if (threadIdx.x == 0) {
@@ -1040,7 +1086,7 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
           u[q] = jq < n ? sc[jq] : 0;
           cnt += jq < n ? 1 : 0;
         }
-        td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
+        td_push_n<WORDS, KIND>(gb, chg, t_cnt, u, cnt, P);
       }
       __syncthreads();  // buffer i & 1 is read: the copy of chunk i + 2 may reuse it
     }
@@ -1067,7 +1113,7 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
           u[i] = ei < b1 ? __ldg(p.col + ei) : 0;
           cnt += ei < b1 ? 1 : 0;
         }
-        td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
+        td_push_n<WORDS, KIND>(gb, chg, t_cnt, u, cnt, P);
       }
     }
   }
@@ -1086,13 +1132,13 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
         u[j] = ej < b1 ? __ldg(p.col + ej) : 0;
         cnt += ej < b1 ? 1 : 0;
       }
-      td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
+      td_push_n<WORDS, KIND>(gb, chg, t_cnt, u, cnt, P);
     }
   }
   // A thread per small vertex; a thin level, whose queue leaves most threads
   // of the team without one, gives it 8 lanes instead, so that its list is
   // one step (32 edges) and not a chain of them.
-  const int lg = (THIN && (long long)nS * 8 <= t.nthreads) ? 3 : 0;
+  const int lg = (KIND == kTdThin && (long long)nS * 8 <= t.nthreads) ? 3 : 0;
   for (long long i0 = t.warp << (5 - lg); i0 < nS; i0 += t.nwarps << (5 - lg)) {
     const long long i = i0 + (t.lane >> lg);
     uint32_t P[WORDS];
@@ -1111,7 +1157,7 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
       const int cnt = (int)max(0LL, min((long long)kTdStep, b1 - e));
 #pragma unroll
       for (int j = 0; j < kTdStep; j++) u[j] = j < cnt ? __ldg(p.col + e + j) : 0;
-      td_push_n<WORDS, THIN>(gb, chg, t_cnt, u, cnt, P);
+      td_push_n<WORDS, KIND>(gb, chg, t_cnt, u, cnt, P);
       e += (long long)kTdStep << lg;
     }
   }
@@ -1121,9 +1167,10 @@ __device__ __forceinline__ void td_run(const Params& p, const GroupBufs& gb, int
 // large levels registers otherwise.
 template <int WORDS, bool STAGE = false>
 __device__ void td_phase(const Params& p, const GroupBufs& gb, int level, const int32_t* qc,
-                         bool thin, const Team& t) {
-  if (thin) td_run<WORDS, false, true>(p, gb, level, qc, t);
-  else td_run<WORDS, STAGE, false>(p, gb, level, qc, t);
+                         int kind, const Team& t) {
+  if (kind == kTdThin) td_run<WORDS, false, kTdThin>(p, gb, level, qc, t);
+  else if (kind == kTdWide) td_run<WORDS, STAGE, kTdWide>(p, gb, level, qc, t);
+  else td_run<WORDS, STAGE, kTdBitmap>(p, gb, level, qc, t);
 }
 
 // Second bottom-up stage: the hubs that were still missing frontier bits

@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(512) k_dl_batch_init(Params p, int g, CondH h_
     ls.sync = 0;
     for (int k = 0; k < kMaxWords; k++) ls.smask[k] = 0u;
     ls.sparse_try = 0;
-    ls.thin = 1;  // level 0: the seeds are its touched list
+    ls.kind = kTdThin;  // level 0: the seeds are its touched list
     ls.have_q = 0;
     ls.t_lvl = ls.t_mid = global_ns();
     cudaGraphSetConditional(h_level, 1u);
@@ -237,7 +237,7 @@ __global__ void DL_INSPECT_BOUNDS k_dl_inspect(Params p, int g, CondH, CondH) {
   const int b = ctl->ls.batch, level = ctl->ls.level;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ls.t_mid = global_ns();
   inspect_phase<WORDS>(p, gb, par_at(ctl, level), dl_batch_size(p, ctl->ls, b), level,
-                       level <= depth_limit(p.db), ctl->ls.thin != 0, ctl->qc[(level + 1) & 1],
+                       level <= depth_limit(p.db), ctl->ls.kind, ctl->qc[(level + 1) & 1],
                        make_team(blockIdx.x, gridDim.x));
 }
 
@@ -289,8 +289,8 @@ __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
   if (!stop) {
     ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
     // a thin level left the next level's queues behind
-    ls.have_q = (nd == kDirTD && ls.thin && ls.dir == kDirTD) ? 1 : 0;
-    ls.thin = (nd == kDirTD && mf <= kThinEdges) ? 1 : 0;
+    ls.have_q = (nd == kDirTD && ls.kind == kTdThin && ls.dir == kDirTD) ? 1 : 0;
+    ls.kind = td_kind(mf, p.v_reach);
     ls.sync = (was_bu && nd == kDirTD) ? 1 : 0;  // top-down needs curr == last again
     ls.dir = nd;
     ls.level = level + 1;
@@ -314,7 +314,7 @@ template <int WORDS>
 __global__ void DL_TD_BOUNDS k_dl_td(Params p, int g, CondH, CondH) {
   const GroupBufs gb = dl_bufs(p, g);
   const int level = gb.ctl->ls.level;
-  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], gb.ctl->ls.thin != 0,
+  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], gb.ctl->ls.kind,
                         make_team(blockIdx.x, gridDim.x));
 }
 

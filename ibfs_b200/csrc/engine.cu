@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(512) k_inspect(Params p, GroupBufs gb, int b, 
   const Team t = make_team(blockIdx.x, gridDim.x);
   const long long k0 = (long long)b * p.C;
   const int n_b = (int)min((long long)p.C, p.n_total - k0);
-  inspect_phase<WORDS>(p, gb, par_at(gb.ctl, level), n_b, level, level <= depth_limit(p.db), false,
+  inspect_phase<WORDS>(p, gb, par_at(gb.ctl, level), n_b, level, level <= depth_limit(p.db), kTdBitmap,
                        nullptr, t);
 }
 
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(512) k_qbuild(Params p, GroupBufs gb, int leve
 template <int WORDS>
 __global__ void __launch_bounds__(512) k_td(Params p, GroupBufs gb, int level) {
   const Team t = make_team(blockIdx.x, gridDim.x);
-  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], false, t);
+  td_phase<WORDS, true>(p, gb, level, gb.ctl->qc[level & 1], kTdBitmap, t);
 }
 
 template <int WORDS>

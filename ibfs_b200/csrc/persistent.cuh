@@ -18,7 +18,7 @@ namespace ibfs {
 // hence how many warps per SM hide the latency of the random gathers.
 template <int WORDS, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
-  __shared__ int s_dir, s_stop, s_err, s_maxl, s_thin;
+  __shared__ int s_dir, s_stop, s_err, s_maxl, s_kind;
   __shared__ int32_t s_rows[kMaxWords * 32];
   const int g = blockIdx.x / p.cpg;
   const Team t = make_team(blockIdx.x % p.cpg, p.cpg);
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
     seed_phase<WORDS, true>(p, gb, p.src + k0, n_b, t);
     BARRIER();
     if (lead) t_mid = global_ns();
-    inspect_phase<WORDS>(p, gb, &ctl->par[0], n_b, 0, true, true, ctl->qc[1], t);
+    inspect_phase<WORDS>(p, gb, &ctl->par[0], n_b, 0, true, kTdThin, ctl->qc[1], t);
     BARRIER();
     int level = 0, cur_dir = kDirTD, max_level = 0, td = 0, bu = 0;
     unsigned long long m_u = (unsigned long long)p.E, teps = 0, prev_changed = 0;
@@ -96,13 +96,13 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
         s_stop = stop;
         s_err = err;
         s_maxl = max_level;
-        s_thin = mf <= kThinEdges ? 1 : 0;
+        s_kind = td_kind(mf, p.v_reach);
       }
       __syncthreads();
       const int stop = s_stop;
       cur_dir = s_dir;
       err = s_err;
-      const bool thin = s_thin != 0 && cur_dir == kDirTD;
+      const int kind = s_kind;
       __syncthreads();
       if (stop) break;
       level++;
@@ -114,12 +114,12 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
           qbuild_phase<WORDS>(p, gb, level, ctl->qc[level & 1], t, after_bu);
           BARRIER();
         }
-        td_phase<WORDS>(p, gb, level, ctl->qc[level & 1], thin, t);
+        td_phase<WORDS>(p, gb, level, ctl->qc[level & 1], kind, t);
         BARRIER();
         if (lead) t_mid = global_ns();
-        inspect_phase<WORDS>(p, gb, par_at(ctl, level), n_b, level, depth_ok, thin,
+        inspect_phase<WORDS>(p, gb, par_at(ctl, level), n_b, level, depth_ok, kind,
                              ctl->qc[(level + 1) & 1], t);
-        have_q = thin;
+        have_q = kind == kTdThin;
         after_bu = false;
       } else {
         // Fused with its inspect work, as in the device loop: the pass writes
