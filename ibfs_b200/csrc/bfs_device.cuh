@@ -563,9 +563,21 @@ __device__ __forceinline__ void zero_plane_if_first(const Params& p, const Group
   }
 }
 
+// Fire-and-forget ORs (red: no value comes back, so nothing waits on them).
+__device__ __forceinline__ void red_or_u32(uint32_t* p, uint32_t x) {
+  asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+__device__ __forceinline__ void red_or_u64(unsigned long long* p, unsigned long long x) {
+  asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+}
+
 // Inspect work of one changed vertex v of level L: new bits, last = curr,
 // counters, planes; deg = its degree.
-template <int WORDS>
+// RED: the planes take the bits as reductions, with nothing to wait for.  A
+// thin level is a chain of dependent accesses, and a read-modify-write per
+// pair of set bits of the level number would be most of it; the other levels
+// move whole lines either way and keep the loads and stores.
+template <int WORDS, bool RED>
 __device__ __forceinline__ void inspect_vertex(const Params& p, const GroupBufs& gb, long long v,
                                                int level, bool depth_ok,
                                                const uint32_t (&full)[WORDS], uint32_t (&fm)[WORDS],
@@ -596,7 +608,21 @@ __device__ __forceinline__ void inspect_vertex(const Params& p, const GroupBufs&
     // planes at a time so that their loads are in flight together.
     uint32_t* q0 = gb.planes + (size_t)v * WORDS;
     unsigned rest = (unsigned)level;
-    while (rest) {
+    while (RED && rest) {
+      const int b0 = __ffs(rest) - 1;
+      rest &= rest - 1;
+      uint32_t* qa = q0 + (size_t)b0 * p.plane_stride;
+      if constexpr (WORDS == 1) {
+        red_or_u32(qa, nb[0]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < WORDS / 2; k++) {
+          const unsigned long long w = ((unsigned long long)nb[2 * k + 1] << 32) | nb[2 * k];
+          if (w) red_or_u64(reinterpret_cast<unsigned long long*>(qa) + k, w);
+        }
+      }
+    }
+    while (!RED && rest) {
       const int b0 = __ffs(rest) - 1;
       rest &= rest - 1;
       uint32_t* qa = q0 + (size_t)b0 * p.plane_stride;
@@ -751,7 +777,8 @@ __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, in
         uint32_t c[WORDS], l[WORDS];
         ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
         ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
-        inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg, c, l);
+        inspect_vertex<WORDS, true>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg,
+                                    c, l);
       }
       q_append(p, gb, qc_next, lane, v, deg, deg_class(p, deg));
     }
@@ -768,8 +795,8 @@ __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, in
         for (int k = 0; k < WORDS; k++) ch |= c[k] != l[k];
         long long deg;
         if (ch)
-          inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps, deg, c,
-                                l);
+          inspect_vertex<WORDS, false>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg, teps,
+                                       deg, c, l);
       }
       const uint32_t bal = __ballot_sync(0xFFFFFFFFu, ch);
       if (lane == 0 && bal) __stcg(chg + (base >> 5), bal);
@@ -783,8 +810,8 @@ __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, in
                      uint32_t c[WORDS], l[WORDS];
                      ld_status<WORDS>(gb.curr + (size_t)v * WORDS, c);
                      ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
-                     inspect_vertex<WORDS>(p, gb, v, level, depth_ok, full, fm, mf, cnt, cdeg,
-                                           teps, deg, c, l);
+                     inspect_vertex<WORDS, false>(p, gb, v, level, depth_ok, full, fm, mf, cnt,
+                                                  cdeg, teps, deg, c, l);
                    }
                  });
   }
@@ -863,14 +890,6 @@ __device__ inline void qbuild_phase(const Params& p, const GroupBufs& gb, int le
       }
     }
   });
-}
-
-// Fire-and-forget ORs (red: no value comes back, so nothing waits on them).
-__device__ __forceinline__ void red_or_u32(uint32_t* p, uint32_t x) {
-  asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
-}
-__device__ __forceinline__ void red_or_u64(unsigned long long* p, unsigned long long x) {
-  asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
 }
 
 // Top-down edges: push the frontier word P of v into neighbours u[0..cnt).

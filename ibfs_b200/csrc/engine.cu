@@ -1231,7 +1231,9 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       void* args[] = {&p};
-      CU(cudaLaunchKernelExC(&cfg, persistent_for(rp.words, occ_level), args));
+      // a grid of at most one CTA per SM runs the 128-register build (level 3)
+      const int build = occ_level == 0 && rp.grid <= g->sms ? 3 : occ_level;
+      CU(cudaLaunchKernelExC(&cfg, persistent_for(rp.words, build), args));
       launches += 1;
     }
     if (capturing) CU(cudaEventRecordWithFlags(g->ev1, cs, cudaEventRecordExternal));

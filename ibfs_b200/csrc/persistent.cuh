@@ -18,7 +18,14 @@ namespace ibfs {
 // hence how many warps per SM hide the latency of the random gathers.
 template <int WORDS, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
-  __shared__ int s_dir, s_stop, s_err, s_maxl, s_kind;
+  // The loop's state that only the decision touches lives here and not in
+  // registers, which the phases need (thread 0 writes it; what every thread
+  // reads alternates by level parity, with a CTA barrier in between).
+  struct LoopShared {
+    unsigned long long m_u[2], prev_changed[2], teps, t_lvl, t_mid;
+    int td, bu, max_level;
+  };
+  __shared__ LoopShared s_loop;
   __shared__ int32_t s_rows[kMaxWords * 32];
   const int g = blockIdx.x / p.cpg;
   const Team t = make_team(blockIdx.x % p.cpg, p.cpg);
@@ -40,7 +47,13 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
   for (int b = g; b < p.nbatches; b += p.G) {
     const long long k0 = (long long)b * p.C;
     const int n_b = (int)min((long long)p.C, p.n_total - k0);
-    unsigned long long t_lvl = global_ns(), t_mid = t_lvl;
+    if (threadIdx.x == 0) {
+      s_loop.m_u[0] = (unsigned long long)p.E;
+      s_loop.prev_changed[0] = 0;
+      s_loop.teps = 0;
+      s_loop.td = s_loop.bu = s_loop.max_level = 0;
+      s_loop.t_lvl = s_loop.t_mid = global_ns();
+    }
     zero_words(gb.last, vpad * WORDS, t);
     zero_words(gb.curr, vpad * WORDS, t);
     zero_words(gb.chg, 2 * p.chg_stride, t);
@@ -53,11 +66,10 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
     BARRIER();
     seed_phase<WORDS, true>(p, gb, p.src + k0, n_b, t);
     BARRIER();
-    if (lead) t_mid = global_ns();
+    if (lead) s_loop.t_mid = global_ns();
     inspect_phase<WORDS>(p, gb, &ctl->par[0], n_b, 0, true, kTdThin, ctl->qc[1], t);
     BARRIER();
-    int level = 0, cur_dir = kDirTD, max_level = 0, td = 0, bu = 0;
-    unsigned long long m_u = (unsigned long long)p.E, teps = 0, prev_changed = 0;
+    int level = 0, cur_dir = kDirTD;
     int err = 0;
     bool have_q = true;     // the queues of the next level are built (by a thin inspect)
     bool after_bu = false;  // the level before was bottom-up: `curr` is one level behind
@@ -66,49 +78,48 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
       // none adds to them before the next barrier
       if (t.block == 0 && threadIdx.x >= 32 && threadIdx.x < 64)
         zero_par(par_at(ctl, level + 2), t.lane);
+      // Every thread takes the decision from the same counters (two 16-byte
+      // loads each), so that no CTA waits for one thread's chain of loads.
+      const Par* pr = par_at(ctl, level);
+      const ulonglong2 c0 = __ldcg(reinterpret_cast<const ulonglong2*>(&pr->changed));
+      const ulonglong2 c1 = __ldcg(reinterpret_cast<const ulonglong2*>(&pr->cdeg));
+      const int range = __ldcg(&pr->range_err);
+      const unsigned long long changed = c0.x, mf = c0.y, cdeg = c1.x;
+      unsigned long long m_u = s_loop.m_u[level & 1];
+      m_u = m_u > cdeg ? m_u - cdeg : 0ull;
+      int stop = 0;
+      if (range) { stop = 1; err = 3; }
+      else if (changed == 0) stop = 1;
+      else if (level + 1 > p.max_levels) { stop = 1; err = 3; }
+      const int nd = choose_dir(level + 1, cur_dir, p.switch_level, p.alpha, p.beta, changed,
+                                s_loop.prev_changed[level & 1], mf, m_u, p.V);
       if (threadIdx.x == 0) {
-        const volatile Par* pr = par_at(ctl, level);
-        const unsigned long long changed = pr->changed, mf = pr->mf, cdeg = pr->cdeg;
-        teps += pr->teps;
-        m_u = m_u > cdeg ? m_u - cdeg : 0ull;
-        int stop = 0;
-        if (pr->range_err) { stop = 1; err = 3; }
-        else if (changed == 0) stop = 1;
-        else if (level + 1 > p.max_levels) { stop = 1; err = 3; }
-        if (changed && !pr->range_err) max_level = level;
-        const int nd = choose_dir(level + 1, cur_dir, p.switch_level, p.alpha, p.beta,
-                                  changed, prev_changed, mf, m_u, p.V);
-        prev_changed = changed;
-        if (t.block == 0) {
+        s_loop.m_u[(level + 1) & 1] = m_u;
+        s_loop.prev_changed[(level + 1) & 1] = changed;
+        s_loop.teps += c1.y;
+        if (changed && !range) s_loop.max_level = level;
+        if (!stop && nd == kDirTD) s_loop.td++;
+        if (!stop && nd != kDirTD) s_loop.bu++;
+        if (lead) {
           if (level < p.lrec_cap) {
             LevelRec r;
             r.batch = b; r.level = level; r.dir = level == 0 ? -1 : cur_dir; r.pad = 0;
             r.frontier = (long long)changed; r.frontier_edges = (long long)mf;
             const unsigned long long t_now = global_ns();
-            r.expand_ns = (long long)(t_mid - t_lvl);
-            r.inspect_ns = (long long)(t_now - t_mid);
-            t_lvl = t_now;
+            r.expand_ns = (long long)(s_loop.t_mid - s_loop.t_lvl);
+            r.inspect_ns = (long long)(t_now - s_loop.t_mid);
+            s_loop.t_lvl = t_now;
             p.lrec[(size_t)b * p.lrec_cap + level] = r;
           }
           if (!stop) ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
         }
-        s_dir = nd;
-        s_stop = stop;
-        s_err = err;
-        s_maxl = max_level;
-        s_kind = td_kind(mf, p.v_reach);
       }
-      __syncthreads();
-      const int stop = s_stop;
-      cur_dir = s_dir;
-      err = s_err;
-      const int kind = s_kind;
-      __syncthreads();
       if (stop) break;
+      cur_dir = nd;
+      const int kind = td_kind(mf, p.v_reach);
       level++;
       const bool depth_ok = level <= depth_limit(p.db);
       if (cur_dir == kDirTD) {
-        td++;
         zero_plane_if_first(p, gb, level, t);
         if (!have_q) {
           qbuild_phase<WORDS>(p, gb, level, ctl->qc[level & 1], t, after_bu);
@@ -116,7 +127,7 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
         }
         td_phase<WORDS>(p, gb, level, ctl->qc[level & 1], kind, t);
         BARRIER();
-        if (lead) t_mid = global_ns();
+        if (lead) s_loop.t_mid = global_ns();
         inspect_phase<WORDS>(p, gb, par_at(ctl, level), n_b, level, depth_ok, kind,
                              ctl->qc[(level + 1) & 1], t);
         have_q = kind == kTdThin;
@@ -124,7 +135,6 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
       } else {
         // Fused with its inspect work, as in the device loop: the pass writes
         // every vertex's new status to `curr`, and the buffers swap roles.
-        bu++;
         Par* par = par_at(ctl, level);
         const Par* prev = par_at(ctl, level - 1);
         const bool filt = bu_filter_level(p.bu_filter, __ldcg(&prev->changed), p.V);
@@ -134,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
         bu_phase<WORDS, true, false>(p, gb, level, prev->fmask, &par->hq_cnt, t, par, n_b,
                                      depth_ok, filt);
         BARRIER();
-        if (lead) t_mid = global_ns();
+        if (lead) s_loop.t_mid = global_ns();
         if (__ldcg(&par->hq_cnt) > 0) {  // same value in every CTA
           bu_defer_phase<WORDS>(p, gb, level, prev->fmask, &par->hq_cnt, t, filt);
           BARRIER();
@@ -158,23 +168,24 @@ __global__ void __launch_bounds__(THREADS, MINB) persistent_kernel(Params p) {
       }
       return;
     }
-    output_phase<WORDS>(p, gb, batch_depth(p, b), s_rows, n_b, s_maxl, t);
+    __syncthreads();  // thread 0's last state
+    output_phase<WORDS>(p, gb, batch_depth(p, b), s_rows, n_b, s_loop.max_level, t);
     if (lead && level + 1 < p.lrec_cap) {
       // one extra record per batch: dir 2 = the output pass
       LevelRec r;
       r.batch = b; r.level = level + 1; r.dir = 2; r.pad = 0;
       r.frontier = 0; r.frontier_edges = 0;
-      r.expand_ns = (long long)(global_ns() - t_lvl);
+      r.expand_ns = (long long)(global_ns() - s_loop.t_lvl);
       r.inspect_ns = 0;
       p.lrec[(size_t)b * p.lrec_cap + level + 1] = r;
     }
     if (lead) {
       BatchRec r;
       r.levels = level;
-      r.max_level = max_level;
-      r.td = td;
-      r.bu = bu;
-      r.teps = teps;
+      r.max_level = s_loop.max_level;
+      r.td = s_loop.td;
+      r.bu = s_loop.bu;
+      r.teps = s_loop.teps;
       r.err = 0;
       r.pad = 0;
       p.brec[b] = r;
