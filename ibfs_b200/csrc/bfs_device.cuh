@@ -1327,6 +1327,16 @@ __device__ __forceinline__ void ld_nbr(const uint32_t* last, const uint32_t* s_h
   else ld_status_ca<WORDS>(last + (size_t)u * WORDS, x);
 }
 
+// A word of shared memory, read again at every use: kept out of registers on
+// purpose (the compiler would hoist a loop-invariant load and spill it).
+__device__ __forceinline__ uint32_t lds_again(const uint32_t* p) {
+  uint32_t x;
+  asm volatile("ld.shared.u32 %0, [%1];"
+               : "=r"(x)
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+  return x;
+}
+
 // A warp ORs the statuses of the neighbours [e0, e_lim) of one vertex into a
 // (the same value in every lane) until no bit of fm is missing; returns
 // whether one still is.  The first step reads 32 neighbours (the highest
@@ -1337,22 +1347,22 @@ template <int WORDS, int HK, bool NC, bool RO>
 __device__ __forceinline__ bool warp_scan(const Params& p, const GroupBufs& gb,
                                           const uint32_t* s_hub, long long hk,
                                           const uint32_t* front, bool filt, int lane,
-                                          long long e0, long long e_lim,
-                                          const uint32_t (&fm)[WORDS], uint32_t (&a)[WORDS]) {
+                                          const int32_t* col, int e0, int e_lim,
+                                          const uint32_t* s_mask, uint32_t (&a)[WORDS]) {
   // gathers in flight per lane; the kernel of its own, whose 42 registers
   // already spill, keeps one (its warps hide the chain)
   constexpr int D = RO ? 1 : WORDS <= 4 ? 4 : 2;
   bool miss = true;
   int width = 32;
-  for (long long e = e0; e < e_lim;) {
+  for (int e = e0; e < e_lim;) {
     uint32_t x[D][WORDS];
 #pragma unroll
     for (int i = 0; i < D; i++) {
 #pragma unroll
       for (int k = 0; k < WORDS; k++) x[i][k] = 0;
-      const long long ei = e + lane + 32 * i;
+      const int ei = e + lane + 32 * i;
       if (32 * i < width && ei < e_lim) {
-        const int32_t u = __ldg(p.col + ei);
+        const int32_t u = __ldg(col + ei);
         if (!filt || in_front<RO>(front, u)) ld_nbr<WORDS, HK, NC>(gb.last, s_hub, hk, u, x[i]);
       }
     }
@@ -1363,13 +1373,18 @@ __device__ __forceinline__ bool warp_scan(const Params& p, const GroupBufs& gb,
 #pragma unroll
       for (int i = 1; i < D; i++) r |= x[i][k];
       a[k] |= __reduce_or_sync(0xFFFFFFFFu, r);
-      miss |= (fm[k] & ~a[k]) != 0u;
+      miss |= (lds_again(s_mask + k) & ~a[k]) != 0u;
     }
     if (!miss) break;
     e += width;
     width = 32 * D;
   }
   return miss;
+}
+
+// Start fetching the line at p into L2 (no register waits for it).
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 // smask (device loop, sparse-source levels): bits pushed top-down after this
@@ -1393,9 +1408,18 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
     for (long long i = threadIdx.x; i < hk * WORDS; i += blockDim.x) s_hub[i] = __ldcg(gb.last + i);
     __syncthreads();
   }
-  uint32_t fm[WORDS];
-#pragma unroll
-  for (int k = 0; k < WORDS; k++) fm[k] = __ldcg(fmask_g + k) & (smask ? ~__ldcg(smask + k) : ~0u);
+  // The frontier mask and the batch's full words stay in shared memory, and
+  // list positions are 32 bits relative to the list: the own-kernel build has
+  // 42 registers a thread (3 x 512 threads per SM), and what does not fit is
+  // spilled inside the sweep.
+  __shared__ uint32_t s_mask[kMaxWords], s_full[kMaxWords], s_fm[kMaxWords];
+  if (threadIdx.x < WORDS) {
+    const int k = threadIdx.x;
+    s_mask[k] = __ldcg(fmask_g + k) & (smask ? ~__ldcg(smask + k) : ~0u);
+    s_full[k] = full_word(n_b, k);
+    s_fm[k] = 0u;  // the OR of the level's new bits
+  }
+  __syncthreads();
   const uint32_t* front = chg_at(gb, p, level - 1);
   uint32_t* out = chg_at(gb, p, level);
   const int lane = t.lane;
@@ -1403,16 +1427,6 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   // are below E < 2^31, so 32 bits hold them
   uint32_t f_mf = 0, f_cnt = 0, f_cdeg = 0;
   unsigned long long f_teps = 0;
-  uint32_t full[WORDS];
-#pragma unroll
-  for (int k = 0; k < WORDS; k++) full[k] = full_word(n_b, k);
-  // the OR of the level's new bits: per warp step a warp OR-reduction into
-  // shared memory (fewer live registers than a per-thread accumulator)
-  __shared__ uint32_t s_fm[kMaxWords];
-  if (FUSED) {
-    if (threadIdx.x < kMaxWords) s_fm[threadIdx.x] = 0u;
-    __syncthreads();
-  }
   const bool first_plane = (level & (level - 1)) == 0;
   const int pb = __ffs(level) - 1;
   bool range = false;
@@ -1422,22 +1436,23 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   for (long long v = t.warp; v < p.big_prefix; v += t.nwarps) {
     uint32_t l[WORDS];
     ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
-    const long long e0 = p.beg[v], e1 = p.beg[v + 1];
+    const long long e0 = p.beg[v];
+    const int deg_v = (int)(p.beg[v + 1] - e0);
     bool need = false;
 #pragma unroll
-    for (int k = 0; k < WORDS; k++) need |= (fm[k] & ~l[k]) != 0u;
-    need = need && e1 > e0;  // uniform across the warp
+    for (int k = 0; k < WORDS; k++) need |= (lds_again(s_mask + k) & ~l[k]) != 0u;
+    need = need && deg_v > 0;  // uniform across the warp
     uint32_t a[WORDS];
 #pragma unroll
     for (int k = 0; k < WORDS; k++) a[k] = l[k];
     bool defer = false;
     if (need) {
-      const long long e_lim = (e1 - e0 > p.hub_t) ? e0 + p.hub_t : e1;
-      const bool miss =
-          warp_scan<WORDS, HK, NC, RO>(p, gb, s_hub, hk, front, filt, lane, e0, e_lim, fm, a);
-      defer = miss && e_lim < e1;
+      const int e_lim = min(deg_v, p.hub_t);
+      const bool miss = warp_scan<WORDS, HK, NC, RO>(p, gb, s_hub, hk, front, filt, lane,
+                                                     p.col + e0, 0, e_lim, s_mask, a);
+      defer = miss && e_lim < deg_v;
       if (defer && lane == 0) {
-        const int nch = (int)((e1 - e_lim + kHubChunk - 1) / kHubChunk);
+        const int nch = (deg_v - e_lim + kHubChunk - 1) / kHubChunk;
         const int base0 = atomicAdd(hq_cnt, nch);
         for (int c = 0; c < nch; c++) gb.hq[base0 + c] = make_int2((int)v, c);
       }
@@ -1461,11 +1476,11 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
         for (int k = 0; k < WORDS; k++) {
           nb[k] = epi ? (a[k] & ~l[k]) : 0u;
           pop += __popc(nb[k]);
-          comp = comp && a[k] == full[k];
+          comp = comp && a[k] == lds_again(s_full + k);
           if (nb[k]) atomicOr(&s_fm[k], nb[k]);
         }
         if (epi) {
-          const uint32_t deg = (uint32_t)(e1 - e0);
+          const uint32_t deg = (uint32_t)deg_v;
           f_cnt += 1;
           f_mf += deg;
           f_teps += (unsigned long long)deg * pop;
@@ -1507,11 +1522,12 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
     const long long v = base + lane;
     const bool valid = v < p.V;
     uint32_t l[WORDS], acc[WORDS];
-    long long b0 = 0, b1 = 0;
+    long long b0 = 0;
+    int deg_v = 0;
     if (valid) {
       ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
       b0 = p.beg[v];
-      b1 = p.beg[v + 1];
+      deg_v = (int)(p.beg[v + 1] - b0);
     } else {
 #pragma unroll
       for (int k = 0; k < WORDS; k++) l[k] = 0;
@@ -1520,43 +1536,49 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
 #pragma unroll
     for (int k = 0; k < WORDS; k++) {
       acc[k] = l[k];
-      need |= (fm[k] & ~l[k]) != 0u;
+      need |= (lds_again(s_mask + k) & ~l[k]) != 0u;
     }
-    need = need && valid && (b1 > b0);
-    const bool small = need && (b1 - b0) <= p.but;
+    need = need && deg_v > 0;
+    const bool small = need && deg_v <= p.but;
+    if (FUSED && need && !first_plane) {
+      // the depth planes that a change of this vertex will read
+      for (unsigned rest = (unsigned)level; rest; rest &= rest - 1)
+        prefetch_l2(gb.planes + (size_t)(__ffs(rest) - 1) * p.plane_stride + (size_t)v * WORDS);
+    }
     // Every vertex that needs bits scans on its own lane first: a small one
     // its whole list, a big one only its first kBuPeek steps -- its
     // highest-degree neighbours, which in the degree order usually cover
     // the frontier bits already.  Only big vertices still missing bits go on
     // to the warp scan below, which takes them one at a time.
     bool covered = false;
-    long long e_big = b0;  // where a big vertex's warp scan starts
+    const int32_t* col = p.col + b0;
+    int e_big = 0;  // where a big vertex's warp scan starts
     if (need) {
       // kBuStep neighbours in flight per step; with col_vec their ids come as
       // aligned 16-byte vectors (col is padded by 4 entries at its end, and
       // a vector is only read when it starts before b1)
       constexpr int S = kBuStep;
-      const int4* col4 = reinterpret_cast<const int4*>(p.col);
-      const long long a0 = p.col_vec ? (b0 & ~3LL) : b0;
-      const long long a_end = small ? b1 : min(b1, a0 + (long long)kBuPeek * S);
-      if (!small) e_big = max(b0, a_end);
-      for (long long a = a0; a < a_end; a += S) {
+      const int a0 = p.col_vec ? -(int)(b0 & 3) : 0;
+      const int a_end = small ? deg_v : min(deg_v, a0 + kBuPeek * S);
+      if (!small) e_big = max(0, a_end);
+      for (int a = a0; a < a_end; a += S) {
         int32_t u[S];
         if (p.col_vec) {
 #pragma unroll
           for (int q = 0; q < S / 4; q++) {
             int4 c4 = make_int4(0, 0, 0, 0);
-            if (q == 0 || a + 4 * q < b1) c4 = __ldg(col4 + ((a >> 2) + q));
+            if (q == 0 || a + 4 * q < deg_v)
+              c4 = __ldg(reinterpret_cast<const int4*>(col + a + 4 * q));
             u[4 * q] = c4.x; u[4 * q + 1] = c4.y; u[4 * q + 2] = c4.z; u[4 * q + 3] = c4.w;
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < S; i++) u[i] = a + i < b1 ? __ldg(p.col + a + i) : 0;
+          for (int i = 0; i < S; i++) u[i] = a + i < deg_v ? __ldg(col + a + i) : 0;
         }
         bool f[S];
 #pragma unroll
         for (int i = 0; i < S; i++) {
-          const bool in = (a + i >= b0) && (a + i < b1);
+          const bool in = (unsigned)(a + i) < (unsigned)deg_v;
           f[i] = in && (!filt || in_front<RO>(front, u[i]));
         }
         uint32_t x[S][WORDS];
@@ -1574,7 +1596,7 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
         for (int k = 0; k < WORDS; k++) {
 #pragma unroll
           for (int i = 0; i < S; i++) acc[k] |= x[i][k];
-          miss |= (fm[k] & ~acc[k]) != 0u;
+          miss |= (lds_again(s_mask + k) & ~acc[k]) != 0u;
         }
         if (!miss) {
           covered = true;
@@ -1588,20 +1610,20 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       const int j = __ffs(big) - 1;
       big &= big - 1;
       const long long e0 = __shfl_sync(0xFFFFFFFFu, b0, j);
-      const long long e1 = __shfl_sync(0xFFFFFFFFu, b1, j);
-      const long long es = __shfl_sync(0xFFFFFFFFu, e_big, j);
+      const int dj = __shfl_sync(0xFFFFFFFFu, deg_v, j);
+      const int es = __shfl_sync(0xFFFFFFFFu, e_big, j);
       uint32_t a[WORDS];
 #pragma unroll
       for (int k = 0; k < WORDS; k++) a[k] = __shfl_sync(0xFFFFFFFFu, acc[k], j);
       // a warp scans at most hub_t neighbours; the rest of a hub that is
       // still missing frontier bits is deferred to bu_defer_phase
       // (the limit counts from the list's start, as bu_defer_phase does)
-      const long long e_lim = (e1 - e0 > p.hub_t) ? e0 + p.hub_t : e1;
-      const bool miss =
-          warp_scan<WORDS, HK, NC, RO>(p, gb, s_hub, hk, front, filt, lane, es, e_lim, fm, a);
-      const bool defer = miss && e_lim < e1;
+      const int e_lim = min(dj, p.hub_t);
+      const bool miss = warp_scan<WORDS, HK, NC, RO>(p, gb, s_hub, hk, front, filt, lane,
+                                                     p.col + e0, es, e_lim, s_mask, a);
+      const bool defer = miss && e_lim < dj;
       if (defer && lane == 0) {
-        const int nch = (int)((e1 - e_lim + kHubChunk - 1) / kHubChunk);
+        const int nch = (dj - e_lim + kHubChunk - 1) / kHubChunk;
         const int base0 = atomicAdd(hq_cnt, nch);
         for (int c = 0; c < nch; c++) gb.hq[base0 + c] = make_int2((int)(base + j), c);
       }
@@ -1629,10 +1651,10 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       for (int k = 0; k < WORDS; k++) {
         nb[k] = epi ? (acc[k] & ~l[k]) : 0u;
         pop += __popc(nb[k]);
-        comp = comp && acc[k] == full[k];
+        comp = comp && acc[k] == lds_again(s_full + k);
       }
       if (epi) {
-        const uint32_t deg = (uint32_t)(b1 - b0);
+        const uint32_t deg = (uint32_t)deg_v;
         f_cnt += 1;
         f_mf += deg;
         f_teps += (unsigned long long)deg * pop;
