@@ -1680,15 +1680,23 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       }
       ch = epi;
     }
+    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, ch);
+    if (!bal) continue;
     if constexpr (FUSED) {
+      // the level's new bits: every source that still expands is in s_fm
+      // after a few ranges, so look before reducing
+      bool more = false;
 #pragma unroll
-      for (int k = 0; k < WORDS; k++) {
-        const uint32_t r = __reduce_or_sync(0xFFFFFFFFu, nb[k]);
-        if (lane == 0 && r) atomicOr(&s_fm[k], r);
+      for (int k = 0; k < WORDS; k++) more |= (nb[k] & ~lds_again(s_fm + k)) != 0u;
+      if (__any_sync(0xFFFFFFFFu, more)) {
+#pragma unroll
+        for (int k = 0; k < WORDS; k++) {
+          const uint32_t r = __reduce_or_sync(0xFFFFFFFFu, nb[k]);
+          if (lane == 0 && r) atomicOr(&s_fm[k], r);
+        }
       }
     }
-    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, ch);
-    if (lane == 0 && bal) atomicOr(out + (base >> 5), bal);
+    if (lane == 0) atomicOr(out + (base >> 5), bal);
   }
   if constexpr (FUSED) {
     if (range) par->range_err = 1;
