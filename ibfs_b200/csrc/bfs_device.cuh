@@ -1558,12 +1558,15 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       // aligned 16-byte vectors (col is padded by 4 entries at its end, and
       // a vector is only read when it starts before b1)
       constexpr int S = kBuStep;
-      const int a0 = p.col_vec ? -(int)(b0 & 3) : 0;
+      // (a list of one step is read id by id: its vector would often straddle
+      // two aligned ones and cost a second step; grid 4096^2 137 -> 133 ms)
+      const bool vec = p.col_vec && deg_v > S;
+      const int a0 = vec ? -(int)(b0 & 3) : 0;
       const int a_end = small ? deg_v : min(deg_v, a0 + kBuPeek * S);
       if (!small) e_big = max(0, a_end);
       for (int a = a0; a < a_end; a += S) {
         int32_t u[S];
-        if (p.col_vec) {
+        if (vec) {
 #pragma unroll
           for (int q = 0; q < S / 4; q++) {
             int4 c4 = make_int4(0, 0, 0, 0);
