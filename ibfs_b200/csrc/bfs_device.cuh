@@ -1433,7 +1433,8 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   // The degree order puts every vertex above the thread-path limit into the
   // prefix [0, p.big_prefix): one warp per vertex there, so that the hubs,
   // which that order packs into a few warps, are spread over all of them.
-  for (long long v = t.warp; v < p.big_prefix; v += t.nwarps) {
+  // (The persistent kernel deals them out to lanes instead, below.)
+  for (long long v = t.warp; RO && v < p.big_prefix; v += t.nwarps) {
     uint32_t l[WORDS];
     ld_status<WORDS>(gb.last + (size_t)v * WORDS, l);
     const long long e0 = p.beg[v];
@@ -1518,9 +1519,17 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
     for (long long i = t.tid; i < n4 + ((p.V - p.v_nz) * WORDS % 4 ? 1 : 0); i += t.nthreads)
       __stcg(q + i, make_uint4(0, 0, 0, 0));
   }
-  for (long long base = start + t.warp * 32; base < p.v_nz; base += rstep) {
-    const long long v = base + lane;
-    const bool valid = v < p.V;
+  // Persistent kernel: the prefix is dealt out like cards, one vertex per lane
+  // and the hubs one per warp, so that the lanes peek at their first
+  // neighbours together and a warp scans only the vertices that are still
+  // missing bits, one after another.  Then the rest, in ranges of 32.
+  const long long deals = RO ? 0 : (p.big_prefix + rstep - 1) / rstep;
+  for (long long it = 0;; it++) {
+    const bool dealt = !RO && it < deals;
+    const long long base = dealt ? 0 : start + t.warp * 32 + (it - deals) * rstep;
+    if (base >= p.v_nz) break;
+    const long long v = dealt ? it * rstep + lane * t.nwarps + t.warp : base + lane;
+    const bool valid = v < (dealt ? p.big_prefix : p.V);
     uint32_t l[WORDS], acc[WORDS];
     long long b0 = 0;
     int deg_v = 0;
@@ -1628,7 +1637,8 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       if (defer && lane == 0) {
         const int nch = (dj - e_lim + kHubChunk - 1) / kHubChunk;
         const int base0 = atomicAdd(hq_cnt, nch);
-        for (int c = 0; c < nch; c++) gb.hq[base0 + c] = make_int2((int)(base + j), c);
+        const int vj = dealt ? (int)(it * rstep + j * t.nwarps + t.warp) : (int)(base + j);
+        for (int c = 0; c < nch; c++) gb.hq[base0 + c] = make_int2(vj, c);
       }
       if (lane == j) {
 #pragma unroll
@@ -1699,7 +1709,11 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
         }
       }
     }
-    if (lane == 0) atomicOr(out + (base >> 5), bal);
+    if (!dealt) {
+      if (lane == 0) atomicOr(out + (base >> 5), bal);
+    } else if (ch) {
+      atomicOr(out + (v >> 5), 1u << (v & 31));
+    }
   }
   if constexpr (FUSED) {
     if (range) par->range_err = 1;
