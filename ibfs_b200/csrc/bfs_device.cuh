@@ -1523,12 +1523,11 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   // and the hubs one per warp, so that the lanes peek at their first
   // neighbours together and a warp scans only the vertices that are still
   // missing bits, one after another.  Then the rest, in ranges of 32.
-  const long long deals = RO ? 0 : (p.big_prefix + rstep - 1) / rstep;
-  for (long long it = 0;; it++) {
-    const bool dealt = !RO && it < deals;
-    const long long base = dealt ? 0 : start + t.warp * 32 + (it - deals) * rstep;
-    if (base >= p.v_nz) break;
-    const long long v = dealt ? it * rstep + lane * t.nwarps + t.warp : base + lane;
+  const long long first = start + t.warp * 32;
+  const long long dealt_v = RO ? 0 : (p.big_prefix + rstep - 1) / rstep * rstep;
+  for (long long base = first - dealt_v; base < p.v_nz; base += rstep) {
+    const bool dealt = !RO && base < start;
+    const long long v = dealt ? base - first + dealt_v + lane * t.nwarps + t.warp : base + lane;
     const bool valid = v < (dealt ? p.big_prefix : p.V);
     uint32_t l[WORDS], acc[WORDS];
     long long b0 = 0;
@@ -1637,7 +1636,8 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       if (defer && lane == 0) {
         const int nch = (dj - e_lim + kHubChunk - 1) / kHubChunk;
         const int base0 = atomicAdd(hq_cnt, nch);
-        const int vj = dealt ? (int)(it * rstep + j * t.nwarps + t.warp) : (int)(base + j);
+        const int vj = dealt ? (int)(base - first + dealt_v + j * t.nwarps + t.warp)
+                             : (int)(base + j);
         for (int c = 0; c < nch; c++) gb.hq[base0 + c] = make_int2(vj, c);
       }
       if (lane == j) {
