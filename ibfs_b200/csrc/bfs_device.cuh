@@ -12,18 +12,19 @@
 // persistent kernel, kernel boundaries in the plain schedule):
 //   expand   top-down push over the joint frontier queues (expander.cuh:
 //            140-331) or bottom-up pull over all vertices (expander.cuh:
-//            341-489); both mark changed vertices in a 1-bit-per-vertex
-//            bitmap (V/8 bytes, L2 resident), double-buffered by level parity
-//            so that the bottom-up pull can skip neighbours outside the
-//            previous frontier;
-//   inspect  walks the bitmap only: new bits = curr & ~last, last = curr,
-//            ORs the new bits into the depth bit-planes of the level number,
-//            and accumulates the direction-switch counters.  Replaces the
-//            O(V) count/scan/gather passes of inspector.cuh:63-525,
-//            scan.cuh:455-655 and the per-level depth_merge writes of
-//            inspector.cuh:8-56,113-120;
-//   qbuild   (only before a top-down level) turns the bitmap into the
-//            small/medium/large queues with warp-ballot compaction
+//            341-489); changed vertices go to a 1-bit-per-vertex bitmap
+//            (V/8 bytes, L2 resident), double-buffered by level parity so
+//            that the bottom-up pull can skip neighbours outside the previous
+//            frontier, and on thin top-down levels also to a list (td_kind);
+//   inspect  takes the changed vertices (from the list, the bitmap or a
+//            sweep): new bits = curr & ~last, last = curr, ORs the new bits
+//            into the depth bit-planes of the level number, and accumulates
+//            the direction-switch counters; bottom-up levels do this work in
+//            the pull itself.  Replaces the O(V) count/scan/gather passes of
+//            inspector.cuh:63-525, scan.cuh:455-655 and the per-level
+//            depth_merge writes of inspector.cuh:8-56,113-120;
+//   qbuild   (only before a top-down level whose queues no thin inspect left
+//            behind) turns the bitmap into the small/medium/large queues
 //            (replaces td_frontier_count/td_frontier_gather).
 // After the last level one pass turns the bit-planes into the depth output
 // (either layout), writing every output byte exactly once.
@@ -167,7 +168,7 @@ struct Params {
   long long v_reach;    // v_nz when no edge points into [v_nz, V) (symmetric
                         // graphs), else V: vertices from v_reach on are reached
                         // only as sources, at depth 0
-  long long big_prefix; // bottom-up: vertices [0, big_prefix) take one warp each
+  long long big_prefix; // bottom-up: vertices [0, big_prefix) are spread over all warps
                         // (degree-ordered graphs: the vertices above the
                         // thread-path limit; a multiple of 32; 0 otherwise)
   int32_t* done_flags;  // per batch, in mapped host memory: 1 once the batch's

@@ -107,7 +107,8 @@ typedef struct ibfs_opts {
     int32_t debug_withhold;/* test hook: CTA 0 never arrives at its first grid
                               barrier, so every wait runs out (IBFS_ERR_TIMEOUT)  */
     int32_t occupancy;     /* persistent kernel register budget / warps per SM:
-                              0: 512 threads x 2 CTAs (64 regs), 1: 256 x 6 (42),
+                              0: 512 threads x 2 CTAs (64 regs; x 1, 128 regs, when
+                              the grid has at most one CTA per SM), 1: 256 x 6 (42),
                               2: 256 x 8 (32), 3: 512 x 1 (128)                 */
     int32_t bu_filter;     /* bottom-up reads a neighbour's status only when the
                               previous frontier bitmap has it (exact: no other
