@@ -170,7 +170,8 @@ struct Params {
                         // only as sources, at depth 0
   long long big_prefix; // bottom-up: vertices [0, big_prefix) are spread over all warps
                         // (degree-ordered graphs: the vertices above the
-                        // thread-path limit; a multiple of 32; 0 otherwise)
+                        // thread-path limit; a multiple of 32, at most V; 0
+                        // otherwise)
   int32_t* done_flags;  // per batch, in mapped host memory: 1 once the batch's
                         // depths are complete in `out` (device loop), so that
                         // the host can stream them out while later batches run

@@ -472,7 +472,9 @@ void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int t
       if (g->dbeg_host[(size_t)mid + 1] - g->dbeg_host[(size_t)mid] > p.but) lo = mid + 1;
       else hi = mid;
     }
-    p.big_prefix = std::min<int64_t>((lo + 31) & ~31LL, (g->V + 31) & ~31LL);
+    // whole ranges only: a last, partial range of big vertices is swept like
+    // the others (the prefix loops index vertices up to big_prefix itself)
+    p.big_prefix = std::min<int64_t>((lo + 31) & ~31LL, g->V & ~31LL);
   }
 }
 
