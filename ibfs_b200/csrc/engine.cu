@@ -661,11 +661,13 @@ static ibfs_status upload_graph(ibfs_graph* g) {
   g->sms = sms;
   ibfs_status s;
   if ((s = g->beg.ensure(sizeof(int64_t) * (size_t)(g->V + 1))) != IBFS_OK) return s;
-  // + 4 entries: the bottom-up reads column ids as aligned 16-byte vectors
-  if ((s = g->col.ensure(sizeof(int32_t) * (size_t)(g->E + 4))) != IBFS_OK) return s;
-  CU(cudaMemset(g->col.p, 0, sizeof(int32_t) * (size_t)(g->E + 4)));
   CU(cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking));
   g->stream = g->own_stream;
+  // + 4 entries: the bottom-up reads column ids as aligned 16-byte vectors.
+  // They are zeroed on the stream that writes the others: a memset on the
+  // default stream is not ordered with a non-blocking stream's kernels.
+  if ((s = g->col.ensure(sizeof(int32_t) * (size_t)(g->E + 4))) != IBFS_OK) return s;
+  CU(cudaMemsetAsync(g->col.as<int32_t>() + g->E, 0, sizeof(int32_t) * 4, g->stream));
   CU(cudaEventCreate(&g->ev0));
   CU(cudaEventCreate(&g->ev1));
   CU(cudaEventCreateWithFlags(&g->ev_out, cudaEventDisableTiming));
