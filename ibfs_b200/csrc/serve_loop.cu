@@ -145,11 +145,14 @@ ibfs_status ServeLoop::init(ibfs_graph* g, const ibfs_opts& o, int G, int slots,
     release();
     return IBFS_ERR_OOM;
   }
-  bool ok = cudaMemcpy(d_groups, hgb.data(), sizeof(GroupBufs) * G_, cudaMemcpyHostToDevice) ==
-                cudaSuccess &&
-            cudaMemset(d_head, 0, sizeof(unsigned long long)) == cudaSuccess;
+  // on the stream that launches the graph: the default stream is not ordered
+  // with it
+  bool ok = cudaMemcpyAsync(d_groups, hgb.data(), sizeof(GroupBufs) * G_, cudaMemcpyHostToDevice,
+                            stream_) == cudaSuccess &&
+            cudaMemsetAsync(d_head, 0, sizeof(unsigned long long), stream_) == cudaSuccess;
   for (int i = 0; ok && i < G_; i++)
-    ok = cudaMemset(hgb[(size_t)i].ctl, 0, sizeof(Ctl)) == cudaSuccess;
+    ok = cudaMemsetAsync(hgb[(size_t)i].ctl, 0, sizeof(Ctl), stream_) == cudaSuccess;
+  ok = ok && cudaStreamSynchronize(stream_) == cudaSuccess;
   if (!ok) {
     (void)cudaGetLastError();
     release();
