@@ -257,6 +257,11 @@ __host__ __device__ inline int td_kind(unsigned long long mf, long long v_reach)
   if (mf <= kThinEdges) return kTdThin;
   return mf * 2 >= (unsigned long long)v_reach ? kTdWide : kTdBitmap;
 }
+// The kind of the next level by its direction: a bottom-up pass marks the
+// bitmap, which is what an inspect step of its own has to walk.
+__host__ __device__ inline int level_kind(int dir, unsigned long long mf, long long v_reach) {
+  return dir == kDirTD ? td_kind(mf, v_reach) : kTdBitmap;
+}
 
 constexpr int kHubScan = 1024;   // neighbours one warp scans before deferring
 constexpr int kHubChunk = 2048;  // edges per deferred chunk (one CTA each)

@@ -290,7 +290,7 @@ __global__ void k_dl_decide(Params p, int g, CondH h_level, CondH h_dir) {
     ctl->qc[level & 1][0] = ctl->qc[level & 1][1] = ctl->qc[level & 1][2] = 0;
     // a thin level left the next level's queues behind
     ls.have_q = (nd == kDirTD && ls.kind == kTdThin && ls.dir == kDirTD) ? 1 : 0;
-    ls.kind = td_kind(mf, p.v_reach);
+    ls.kind = level_kind(nd, mf, p.v_reach);
     ls.sync = (was_bu && nd == kDirTD) ? 1 : 0;  // top-down needs curr == last again
     ls.dir = nd;
     ls.level = level + 1;
