@@ -219,11 +219,19 @@ struct ibfs_graph {
   int32_t* d_done = nullptr;
   size_t done_cap = 0;
   cudaEvent_t ev_out = nullptr;
-  // device-loop graphs, keyed by the launch Params: a few entries, because a
-  // server's rounds alternate between group counts (1..4 batches per round)
-  static constexpr int kDlCache = 4;
+  // device-loop graphs, keyed by the launch Params.  Runs of any source count
+  // share one per status word count and group count: one batch takes 1, 2, 4
+  // or 8 words and one group, more batches the width's words and up to four
+  // groups, so eight entries hold every run of one set of options.
+  static constexpr int kDlCache = 8;
   GraphCache dlcache[kDlCache];
   unsigned dl_next = 0;
+  int64_t dl_builds = 0;
+  // the largest device-loop run so far (or these sizes): what its run block is
+  // laid out for, so that the sources' and rows' addresses (baked into the
+  // graphs) stay put
+  int dl_groups = 4, dl_batches = 128;
+  int64_t dl_sources = 1024;
   std::mutex mu;
 };
 
@@ -338,9 +346,9 @@ static cudaError_t launch_plain_output(const Params& p, const GroupBufs& gb, int
 }
 
 // Byte offsets inside the run block: group table, control blocks, batch
-// records, sources, output rows.  The capacities are powers of two, so that the
-// addresses (baked into cached CUDA graphs) stay put across runs of similar
-// size.
+// records, sources, output rows.  The capacities are powers of two; the device
+// loop's are those of its largest run so far, so that the addresses (baked into
+// cached CUDA graphs) move only when a run outgrows every earlier one.
 struct RunBlock {
   size_t groups, ctl, brec, src, row, bytes;
   RunBlock(int G, int nbatches, int64_t n) {
@@ -485,6 +493,9 @@ void set_output_params(const ibfs_graph* g, int C, uint8_t* dout, Params* p) {
               : (g->V % 4 == 0 && (reinterpret_cast<uintptr_t>(dout) & 3) == 0) ? 4
                                                                                : 0;
 }
+
+// Device-loop graphs this handle has built (tests; not part of the C ABI).
+extern "C" int64_t ibfs_internal_graph_builds(const ibfs_graph* g) { return g->dl_builds; }
 
 int graph_sms(const ibfs_graph* g) { return g->sms; }
 int64_t graph_defer_cap(const ibfs_graph* g) { return g->defer_cap; }
@@ -1072,7 +1083,13 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   }
   const bool dev_gb = o.groupby == 2 && !rows_in;
   ibfs_status bs;
-  const RunBlock rb(rp.G, rp.nbatches, n);
+  if (devloop) {
+    g->dl_groups = std::max(g->dl_groups, rp.G);
+    g->dl_batches = std::max(g->dl_batches, rp.nbatches);
+    g->dl_sources = std::max(g->dl_sources, n);
+  }
+  const RunBlock rb = devloop ? RunBlock(g->dl_groups, g->dl_batches, g->dl_sources)
+                              : RunBlock(rp.G, rp.nbatches, n);
   if ((bs = g->h_run.ensure(rb.bytes)) != IBFS_OK) return bs;
   if ((bs = g->d_run.ensure(rb.bytes)) != IBFS_OK) return bs;
   uint8_t* const hrun = g->h_run.as<uint8_t>();
@@ -1328,6 +1345,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
       }
       slot->exec = exec;
       slot->key = key;
+      g->dl_builds++;
     }
     if (rp.host_out && dev_gb) {
       // the device GroupBy chose the rows: the sink needs them on the host
