@@ -1225,10 +1225,12 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   }
 
   // Depths of a persistent run to host memory: from 1 MB on through the sink
-  // (direct when pinned, its staging ring when pageable).  R-MAT scale 12 to
-  // a reused pageable array, one driver copy / ring: 0.5 MB 213 / 214 us,
-  // 1 MB 260 / 217 us, 2 MB 326 / 243 us, 8 MB 715 / 471 us per call.
-  const bool staged = persistent && rp.host_out && !use_graph && out_bytes >= (1u << 20);
+  // (direct when pinned, its staging ring when pageable and the ring pays).
+  // R-MAT scale 12 to a reused pageable array, one driver copy / ring: 0.5 MB
+  // 213 / 214 us, 1 MB 260 / 217 us, 2 MB 326 / 243 us, 8 MB 715 / 471 us per
+  // call.
+  const bool staged = persistent && rp.host_out && !use_graph && out_bytes >= (1u << 20) &&
+                      (DepthSink::is_pinned(depth_out) || g->sink.ring_pays(out_bytes));
 
   auto enqueue = [&](cudaStream_t cs, bool capturing) -> ibfs_status {
     {
@@ -1300,10 +1302,14 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
       ibfs_status es2 = enqueue(s, false);
       if (es2 != IBFS_OK) return es2;
       if (staged) {
-        CU(g->sink.begin(g->device, depth_out, dout));
-        CU(g->sink.wait_for(g->ev1));
-        CU(g->sink.push(0, out_bytes));
-        CU(g->sink.finish());
+        if (g->sink.begin(g->device, depth_out, dout) == cudaSuccess) {
+          CU(g->sink.wait_for(g->ev1));
+          CU(g->sink.push(0, out_bytes));
+          CU(g->sink.finish());
+        } else {  // no memory to pin: the driver's copy needs none
+          (void)cudaGetLastError();
+          CU(cudaMemcpyAsync(depth_out, dout, out_bytes, cudaMemcpyDeviceToHost, s));
+        }
       }
     }
   } else if (devloop) {

@@ -217,22 +217,33 @@ class DepthSink {
   void release();
   size_t copied() const { return copied_; }
   bool pinned() const { return pinned_; }
+  static bool is_pinned(const void* p);
+  // whether a run of `bytes` that has the choice should take the staging ring
+  bool ring_pays(size_t bytes);
 
  private:
   static constexpr int kSlots = 8;
   static constexpr size_t kSlotBytes = 4u << 20;
+  static constexpr size_t kRingPays = 32u << 20;
+  static constexpr size_t kHuge = 2u << 20;  // the ring starts on a huge page
+  static constexpr size_t kMapBytes = kSlots * kSlotBytes + kHuge;
   struct Piece {
     size_t off, at, bytes;  // output offset, offset in the slot, length
   };
   struct Slot {
-    void* buf = nullptr;
+    uint8_t* buf = nullptr;  // into ring_
     cudaEvent_t ev = nullptr;
     std::vector<Piece> pieces;
   };
+  cudaError_t make_ring();
   cudaError_t drain_one();
   cudaError_t close_open();
   int device_ = -1;
   cudaStream_t stream_ = nullptr;
+  uint8_t* map_ = nullptr;   // the mapping that holds the ring
+  uint8_t* ring_ = nullptr;  // kSlots slots, registered with CUDA
+  bool registered_ = false;
+  size_t unpaid_ = 0;  // bytes of the runs that went without the ring
   std::vector<Slot> slots_;
   std::vector<int> pending_;  // closed slots in copy order
   int next_ = 0;

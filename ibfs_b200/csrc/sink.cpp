@@ -16,8 +16,13 @@
 //     faults of a fresh buffer in parallel.  512 rows of 4,194,304 depths
 //     (2.1 GB) from R-MAT scale 22 to a fresh / a reused pageable array: 429 /
 //     253 ms with four 32 MiB slots spread row by row once all were full, 158
-//     to 184 / 58 ms now.
+//     to 184 / 58 ms now.  The slots are one huge-page block, touched by all
+//     cores and registered once: 1.7 to 2.5 ms to make and 1 to 1.5 to free, where
+//     eight pinned allocations took 15 to 24 and 5.
+#include <sys/mman.h>
+
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <vector>
 
@@ -27,7 +32,7 @@
 
 namespace ibfs {
 
-static bool is_pinned(const void* p) {
+bool DepthSink::is_pinned(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -39,11 +44,13 @@ static bool is_pinned(const void* p) {
 DepthSink::~DepthSink() { release(); }
 
 void DepthSink::release() {
-  for (auto& s : slots_) {
-    if (s.buf) cudaFreeHost(s.buf);
+  for (auto& s : slots_)
     if (s.ev) cudaEventDestroy(s.ev);
-  }
   slots_.clear();
+  if (registered_) cudaHostUnregister(ring_);
+  registered_ = false;
+  if (map_) munmap(map_, kMapBytes);
+  map_ = ring_ = nullptr;
   if (stream_) cudaStreamDestroy(stream_);
   stream_ = nullptr;
   device_ = -1;
@@ -66,17 +73,54 @@ cudaError_t DepthSink::begin(int device, void* dst_host, const uint8_t* src_dev)
   }
   pinned_ = is_pinned(dst_host);
   if (!pinned_ && slots_.empty()) {
-    slots_.resize(kSlots);
-    for (auto& sl : slots_) {
-      cudaError_t e = cudaMallocHost(&sl.buf, kSlotBytes);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming);
-      if (e != cudaSuccess) {
-        release();
-        return e;
-      }
+    const cudaError_t e = make_ring();
+    if (e != cudaSuccess) {
+      release();
+      return e;
     }
   }
   return cudaSuccess;
+}
+
+// The block is a mapping of its own that a forked child does not inherit: a
+// page shared with a child would be copied on the next write and leave the
+// registration on the old one.
+cudaError_t DepthSink::make_ring() {
+  constexpr size_t kBytes = kSlots * kSlotBytes;
+  void* m = mmap(nullptr, kMapBytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  if (m == MAP_FAILED) return cudaErrorMemoryAllocation;
+  map_ = static_cast<uint8_t*>(m);
+  ring_ = map_ + (kHuge - reinterpret_cast<uintptr_t>(map_) % kHuge) % kHuge;
+  (void)madvise(ring_, kBytes, MADV_HUGEPAGE);
+  (void)madvise(ring_, kBytes, MADV_DONTFORK);
+#pragma omp parallel for schedule(static)
+  for (long long i = 0; i < (long long)(kBytes / kHuge); i++)
+    std::memset(ring_ + (size_t)i * kHuge, 0, kHuge);
+  cudaError_t e = cudaHostRegister(ring_, kBytes, cudaHostRegisterDefault);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return e;
+  }
+  registered_ = true;
+  slots_.resize(kSlots);
+  for (int i = 0; i < kSlots; i++) {
+    slots_[i].buf = ring_ + i * kSlotBytes;
+    e = cudaEventCreateWithFlags(&slots_[i].ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// A run whose depths could as well go by one driver copy takes the ring once
+// there is one, and makes one when it sends kRingPays bytes or when the runs
+// before it have sent as many without: making and freeing the ring costs
+// about 3 ms, what it saves is 0.03 to 0.04 ms per MB to a reused array and 0.15
+// per MB to one whose pages are fresh (those of 32 MB and more, which malloc
+// maps anew), so a program that opens a graph, takes a few small results and
+// leaves does not pay for it.
+bool DepthSink::ring_pays(size_t bytes) {
+  if (slots_.empty() && unpaid_ < kRingPays) unpaid_ += bytes;
+  return !slots_.empty() || unpaid_ >= kRingPays;
 }
 
 cudaError_t DepthSink::wait_for(cudaEvent_t ev) {
@@ -103,7 +147,7 @@ cudaError_t DepthSink::drain_one() {
                                [](size_t x, const Piece& pc) { return x < pc.at + pc.bytes; });
     for (; it != sl.pieces.end() && it->at < hi; ++it) {
       const size_t a = std::max(lo, it->at), b = std::min(hi, it->at + it->bytes);
-      std::memcpy(dst_ + it->off + (a - it->at), static_cast<const uint8_t*>(sl.buf) + a, b - a);
+      std::memcpy(dst_ + it->off + (a - it->at), sl.buf + a, b - a);
     }
   }
   sl.pieces.clear();
@@ -150,7 +194,7 @@ cudaError_t DepthSink::push(size_t off, size_t bytes) {
     }
     const size_t n = std::min(bytes, kSlotBytes - fill_);
     Slot& sl = slots_[open_];
-    const cudaError_t e = cudaMemcpyAsync(static_cast<uint8_t*>(sl.buf) + fill_, src_ + off, n,
+    const cudaError_t e = cudaMemcpyAsync(sl.buf + fill_, src_ + off, n,
                                           cudaMemcpyDeviceToHost, stream_);
     if (e != cudaSuccess) return e;
     sl.pieces.push_back({off, fill_, n});
