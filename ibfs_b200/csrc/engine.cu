@@ -269,17 +269,6 @@ static ibfs_status check_opts(const ibfs_opts* o) {
   return IBFS_OK;
 }
 
-// Per-group workspace bytes for (V, W, C, db).
-static size_t group_bytes(int64_t V, int64_t E, int words, int C, int db, int lrg, int chunk,
-                          bool /*unused*/) {
-  const size_t vpad = (size_t)((V + 31) & ~31LL);
-  const size_t nchg = (size_t)(((V + 31) / 32 + 127) & ~127LL);
-  const size_t capl = (size_t)(E / std::max(chunk, 1) + std::min<int64_t>(V, E / std::max(lrg, 1)) + 16);
-  size_t b = 2 * vpad * words * 4 + nchg * 4 + 2 * (size_t)V * 4 + capl * 8 + sizeof(Ctl);
-  b += (size_t)(db == 1 ? 8 : 16) * vpad * words * 4 + nchg * 4;  // planes + 2nd bitmap
-  return b;
-}
-
 // Occupancy levels of the persistent kernel: threads per CTA; the CTAs per
 // SM its register budget is sized for are 2, 6, 8 and 1 (the template
 // arguments below).
@@ -397,6 +386,26 @@ static size_t group_layout(const ibfs_graph* g, int words, int db, int lrg, int 
   gb->ql = reinterpret_cast<int2*>(take(capl * 8));
   gb->hq = reinterpret_cast<int2*>(take((size_t)g->defer_cap * 8));
   return off;
+}
+
+// The number of groups, at most G, whose workspaces have to grow by no more
+// than half of the free device memory.  What a group holds already counts: a
+// handle's runs differ in the status words they keep.
+static int groups_that_fit(const ibfs_graph* g, const RunPlan& rp, const ibfs_opts& o, int G) {
+  GroupBufs gb;
+  const size_t per = group_layout(g, rp.words, rp.db, o.lrg_shed, rp.threads * 4, nullptr, &gb);
+  auto growth = [&](int groups) {
+    size_t b = 0;
+    for (int i = 0; i < groups; i++) {
+      const size_t have = i < (int)g->groups.size() ? g->groups[i].mem.bytes : 0;
+      b += per > have ? per - have : 0;
+    }
+    return b;
+  };
+  size_t freeb = 0, totb = 0;
+  if (G <= 1 || growth(G) == 0 || cudaMemGetInfo(&freeb, &totb) != cudaSuccess) return G;
+  while (G > 1 && growth(G) > freeb / 2) G--;
+  return G;
 }
 
 // Allocate / reuse the workspace for G groups.
@@ -1036,14 +1045,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
       // a graph that fills the GPU by itself (team_ctas) takes four at most
       if (g->E / 12288 >= total_ctas) G = std::min(G, 4);
       while (G > 1 && (int64_t)((rp.nbatches + G - 1) / G) * G * 100 > (int64_t)rp.nbatches * 115) G--;
-      // memory guard (only when the workspace has to grow to G groups)
-      size_t freeb = 0, totb = 0;
-      if ((int)g->groups.size() < G && cudaMemGetInfo(&freeb, &totb) == cudaSuccess) {
-        const size_t per = group_bytes(g->V, g->E, rp.words, rp.C, db, o.lrg_shed, rp.threads * 4,
-                                       false);
-        const size_t budget = (size_t)(freeb * 0.5);
-        G = (int)std::max<size_t>(1, std::min<size_t>((size_t)G, budget / std::max<size_t>(per, 1)));
-      }
+      G = groups_that_fit(g, rp, o, G);
     }
     G = std::max(1, std::min(G, std::min(rp.nbatches, total_ctas)));
     rp.G = G;
@@ -1054,15 +1056,8 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
     // concurrent batches are parallel branches of the graph; each kernel is
     // sized by its own occupancy, so groups only overlap one batch's serial
     // stretches (decisions, small levels) with another's work
-    int G = std::min(o.groups ? o.groups : 4, rp.nbatches);  // 4: best on R-MAT s22-24
-    size_t freeb = 0, totb = 0;
-    if (G > 1 && (int)g->groups.size() < G && cudaMemGetInfo(&freeb, &totb) == cudaSuccess) {
-      const size_t per = group_bytes(g->V, g->E, rp.words, rp.C, db, o.lrg_shed, rp.threads * 4,
-                                     false);
-      G = (int)std::max<size_t>(1, std::min<size_t>((size_t)G, (size_t)(freeb * 0.5) /
-                                                                  std::max<size_t>(per, 1)));
-    }
-    rp.G = std::max(1, std::min(G, rp.nbatches));
+    const int G = std::min(o.groups ? o.groups : 4, rp.nbatches);  // 4: best on R-MAT s22-24
+    rp.G = groups_that_fit(g, rp, o, G);
     rp.cpg = total_ctas;
     rp.grid = total_ctas;
   } else {
