@@ -123,6 +123,7 @@ struct DevBuf {
     if (e != cudaSuccess) {
       p = nullptr;
       last_cuda_error() = e;
+      (void)cudaGetLastError();  // reported here: leave none to the program's own checks
       return IBFS_ERR_OOM;
     }
     bytes = std::max<size_t>(want, 256);
@@ -153,6 +154,7 @@ struct PinBuf {
     bytes = 0;
     if (cudaMallocHost(&p, std::max<size_t>(want, 256)) != cudaSuccess) {
       p = nullptr;
+      (void)cudaGetLastError();
       return IBFS_ERR_OOM;
     }
     bytes = std::max<size_t>(want, 256);
