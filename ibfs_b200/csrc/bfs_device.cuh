@@ -266,6 +266,16 @@ __host__ __device__ inline int level_kind(int dir, unsigned long long mf, long l
 constexpr int kHubScan = 1024;   // neighbours one warp scans before deferring
 constexpr int kHubChunk = 2048;  // edges per deferred chunk (one CTA each)
 
+// Bottom-up positions inside one list are 32 bits (registers are what the
+// sweep is short of: 64-bit ones cost the grid and the 256-bit runs 2 %).  Only
+// a list with duplicates can be longer than kListMax, which leaves room for a
+// step of 128 past the end; a graph that has one runs every level top-down,
+// where positions are 64 bits.
+constexpr long long kListMax = 0x7FFFF000;
+__host__ __device__ inline int switch_level_for(int switch_level, long long max_deg) {
+  return max_deg > kListMax ? 0x7FFFFFFF : switch_level;
+}
+
 // Neighbour statuses of a bottom-up pass that runs as a kernel of its own
 // (RO: nothing writes `last` while it runs) are read through L1 (ld.global.nc):
 // most gathers hit the few hub words that the degree order packs into the
@@ -1430,10 +1440,18 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   const uint32_t* front = chg_at(gb, p, level - 1);
   uint32_t* out = chg_at(gb, p, level);
   const int lane = t.lane;
-  // FUSED counters (as inspect_phase); degree sums of one thread's vertices
-  // are below E < 2^31, so 32 bits hold them
+  // FUSED counters (as inspect_phase).  A degree is below 2^31 here; a sum of
+  // one thread's degrees passes 2^32 only in a graph of that many edges, and
+  // then hands the carry to the level's -- in the persistent kernel, whose team
+  // may be one CTA.  The own-kernel pass has the whole GPU's threads, so one of
+  // them would have to own lists of 2^32 edges; these two sums only steer the
+  // direction choice, and the carry costs its sweep 1.5 % (grid 4096^2).
   uint32_t f_mf = 0, f_cnt = 0, f_cdeg = 0;
   unsigned long long f_teps = 0;
+  auto add_degree = [](uint32_t* sum, uint32_t deg, unsigned long long* total) {
+    *sum += deg;
+    if (!RO && *sum < deg) atomicAdd(total, 1ull << 32);
+  };
   const bool first_plane = (level & (level - 1)) == 0;
   const int pb = __ffs(level) - 1;
   bool range = false;
@@ -1490,9 +1508,9 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
         if (epi) {
           const uint32_t deg = (uint32_t)deg_v;
           f_cnt += 1;
-          f_mf += deg;
+          add_degree(&f_mf, deg, &par->mf);
           f_teps += (unsigned long long)deg * pop;
-          if (comp) f_cdeg += deg;
+          if (comp) add_degree(&f_cdeg, deg, &par->cdeg);
           if (!depth_ok) range = true;
           atomicOr(out + (v >> 5), 1u << (v & 31));
         }
@@ -1676,9 +1694,9 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       if (epi) {
         const uint32_t deg = (uint32_t)deg_v;
         f_cnt += 1;
-        f_mf += deg;
+        add_degree(&f_mf, deg, &par->mf);
         f_teps += (unsigned long long)deg * pop;
-        if (comp) f_cdeg += deg;
+        if (comp) add_degree(&f_cdeg, deg, &par->cdeg);
         if (!depth_ok) range = true;
       }
       uint32_t* q0 = gb.planes + (size_t)v * WORDS;

@@ -446,7 +446,7 @@ void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int t
   p.lrg = o.lrg_shed;
   p.chunk = threads * 4;
   p.but = o.bu_thread_max > 0 ? o.bu_thread_max : 32;
-  p.switch_level = o.switch_level;
+  p.switch_level = switch_level_for(o.switch_level, g->max_deg);
   p.alpha = o.alpha;
   p.beta = o.beta;
   p.max_levels = o.max_levels ? o.max_levels : 65534;

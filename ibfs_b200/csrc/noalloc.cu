@@ -50,6 +50,15 @@ ibfs_status scratch_base(unsigned char** out) {
   return IBFS_OK;
 }
 
+// The largest degree of the caller's CSR, which lives on the device only.
+__global__ void k_max_degree(const int64_t* beg, int64_t V, unsigned long long* out) {
+  unsigned long long m = 0;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
+       v += (int64_t)gridDim.x * blockDim.x)
+    m = max(m, (unsigned long long)(beg[v + 1] - beg[v]));
+  atomicMax(out, m);
+}
+
 }  // namespace
 
 using namespace ibfs;
@@ -118,6 +127,17 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   gb.ql = reinterpret_cast<int2*>(base + o_ql);
   gb.hq = nullptr;
   gb.ctl = reinterpret_cast<Ctl*>(base + o_ctl);
+  // A list too long for bottom-up positions needs more than that many edges;
+  // the records' place serves as scratch.
+  unsigned long long max_deg = 0;
+  if (E > kListMax) {
+    unsigned long long* d_max = reinterpret_cast<unsigned long long*>(base + o_brec);
+    NA_CU(cudaMemsetAsync(d_max, 0, sizeof(max_deg), s));
+    k_max_degree<<<128, 256, 0, s>>>(beg_dev, V, d_max);
+    NA_CU(cudaGetLastError());
+    NA_CU(cudaMemcpyAsync(&max_deg, d_max, sizeof(max_deg), cudaMemcpyDeviceToHost, s));
+    NA_CU(cudaStreamSynchronize(s));
+  }
   // What must start at zero: the control block (barrier, error, counters)
   // and the batch records.  Status words and bitmap are cleared per batch by
   // the kernel itself.
@@ -155,7 +175,7 @@ extern "C" ibfs_status ibfs_run_static_scratch(const int64_t* beg_dev, const int
   p.lrg = lrg;
   p.chunk = chunk;
   p.but = 32;
-  p.switch_level = -1;
+  p.switch_level = switch_level_for(-1, (long long)max_deg);
   p.alpha = 14.0f;
   p.beta = 24.0f;
   p.max_levels = 254;

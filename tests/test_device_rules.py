@@ -39,3 +39,19 @@ def test_level_kind(tmp_path):
     CHECK(level_kind(kDirBU, mf[i], V) == kTdBitmap);
   }
 """)
+
+
+def test_long_lists_run_top_down(tmp_path):
+    """A degree that 32-bit list positions do not hold turns every level
+    top-down, whatever switch level was asked for; other graphs keep theirs."""
+    run_checks(tmp_path, """
+  for (int sw : {-1, 0, 3, 1000}) {
+    for (long long d : {0ll, 33ll, 0x7FFFF000ll}) CHECK(switch_level_for(sw, d) == sw);
+    for (long long d : {0x7FFFF001ll, 0x7FFFFFFFll, 0x80000000ll, 0x100000010ll}) {
+      const int s = switch_level_for(sw, d);
+      for (int level : {1, 2, 65535})
+        CHECK(choose_dir(level, kDirTD, s, 4.0f, 24.0f, 9, 1, 1ull << 40, 1, 10) == kDirTD);
+    }
+  }
+  CHECK(kListMax + 128 <= 0x7FFFFFFF);
+""")
