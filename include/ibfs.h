@@ -119,7 +119,9 @@ typedef struct ibfs_opts {
                               thread each; above it a warp scans (0: 32)          */
     int32_t td_stage;      /* 1: top-down stages each large vertex's adjacency
                               chunk in shared memory by double-buffered bulk
-                              (TMA) copies (plain and device-loop schedules);
+                              (TMA) copies (plain and device-loop schedules; the
+                              device loop's levels of at most 2^20 frontier edges
+                              have few chunks and read them directly);
                               0 (default): reads the chunk directly              */
     int32_t sparse_push;   /* device loop: d > 0 makes a bottom-up level that
                               follows a top-down one push, top-down, the sources
