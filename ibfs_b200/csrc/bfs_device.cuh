@@ -281,8 +281,9 @@ __host__ __device__ inline int switch_level_for(int switch_level, long long max_
 // most gathers hit the few hub words that the degree order packs into the
 // first lines of `last`, and L1 serves them instead of L2.  Measured on
 // R-MAT scale 24, one batch at a time: bottom-up 25.1 -> 19.4 ms per
-// 1024-source run; the persistent kernel, whose other phases write `last`
-// within the same launch, keeps L2 reads.
+// 1024-source run.  The persistent kernel, whose other phases write `last`
+// within the same launch, must not use that path; its sweep reads `last` by
+// ordinary cached loads (ld_status_ca), its deferred hub chunks through L2.
 #ifndef IBFS_BU_NC
 #define IBFS_BU_NC 1
 #endif
@@ -355,8 +356,8 @@ __device__ __forceinline__ void ld_status_nc(const uint32_t* p, uint32_t (&x)[WO
   }
 }
 
-// Status read through L1 inside the persistent kernel, for a buffer that no
-// thread writes during the phase: the team barrier before the phase (release
+// Status read through L1 inside the persistent kernel, only for a buffer that
+// no thread writes during the phase: the team barrier before the phase (release
 // by every CTA, acquire by every CTA, then a CTA barrier) makes the earlier
 // writes visible to ordinary cached loads.
 template <int WORDS>
@@ -760,14 +761,14 @@ __device__ __forceinline__ void q_append(const Params& p, const GroupBufs& gb, i
 }
 
 // ---------------------------------------------------------------------------
-// Phase: inspect level L.  Fixes last, updates the depth bit-planes and the
-// counters of every changed vertex, which it takes
-// vertices from the list, the bitmap or a sweep (td_kind).  What bounds a thin level is its chain of dependent L2 reads (queue entry,
-// offsets, column id, status, then list entry, statuses, planes), so the
-// step is one vertex per lane and 8 lanes per pushed small vertex.  A
-// 256 x 1024 grid without shortcuts (64 sources, 1269 levels, about 12,500
-// vertices each) went from 144 to 34 ms when its levels stopped walking the
-// whole bitmap with a few warps.
+// Phase: inspect level L.  Takes the changed vertices from the list, the
+// bitmap or a sweep (td_kind), fixes last, and updates the depth bit-planes
+// and the counters.  What bounds a thin level is its chain of dependent L2
+// reads (queue entry, offsets, column id, status, then list entry, statuses,
+// planes), so the step is one vertex per lane and 8 lanes per pushed small
+// vertex.  A 256 x 1024 grid without shortcuts (64 sources, 1269 levels, about
+// 12,500 vertices each) went from 144 to 34 ms when its levels stopped walking
+// the whole bitmap with a few warps.
 // ---------------------------------------------------------------------------
 template <int WORDS>
 __device__ void inspect_phase(const Params& p, const GroupBufs& gb, Par* par, int n_b,
@@ -1310,7 +1311,7 @@ __device__ void bu_defer_phase(const Params& p, const GroupBufs& gb, int level,
 // (sw_expand_warp, expander.cuh:341-422).
 // ---------------------------------------------------------------------------
 //
-// FUSED (device loop only) also does the inspect work of the level in the
+// FUSED (device loop and persistent kernel) also does the inspect work of the level in the
 // same pass, so that bottom-up levels need no inspect pass: every vertex's
 // new status goes to `curr` (for all vertices, changed or not: `curr` then
 // holds the complete status of the level while `last` keeps the previous
@@ -1319,6 +1320,7 @@ __device__ void bu_defer_phase(const Params& p, const GroupBufs& gb, int level,
 // 2^b, so it needs no zeroing), and the changed bitmap is still marked for a
 // following top-down level.  Hubs deferred to bu_defer_phase get their
 // planes and counters in bu_hub_epilogue.
+
 // Status of neighbour u for a bottom-up scan: from the CTA's shared-memory
 // copy of the hubs' statuses when u is one of the first hk vertices, else
 // from `last`, which no thread writes during the pass (through L1: the
@@ -1366,7 +1368,7 @@ __device__ __forceinline__ bool warp_scan(const Params& p, const GroupBufs& gb,
                                           const uint32_t* front, bool filt, int lane,
                                           const int32_t* col, int e0, int e_lim,
                                           const uint32_t* s_mask, uint32_t (&a)[WORDS]) {
-  // gathers in flight per lane; the kernel of its own, whose 42 registers
+  // gathers in flight per lane; the kernel of its own, whose 40 registers
   // already spill, keeps one (its warps hide the chain)
   constexpr int D = RO ? 1 : WORDS <= 4 ? 4 : 2;
   bool miss = true;
@@ -1427,7 +1429,7 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   }
   // The frontier mask and the batch's full words stay in shared memory, and
   // list positions are 32 bits relative to the list: the own-kernel build has
-  // 42 registers a thread (3 x 512 threads per SM), and what does not fit is
+  // 40 registers a thread (3 x 512 threads per SM), and what does not fit is
   // spilled inside the sweep.
   __shared__ uint32_t s_mask[kMaxWords], s_full[kMaxWords], s_fm[kMaxWords];
   if (threadIdx.x < WORDS) {
@@ -2063,23 +2065,6 @@ __device__ void push_run_phase(const Params& p, const GroupBufs& gb, Par* par, i
 __device__ __forceinline__ uint32_t nib_to_bytes(uint32_t nib) {
   return (nib * 0x00204081u) & 0x01010101u;
 }
-// 8 bits -> every 4th bit of a word (bit r -> bit 4r).
-__device__ __forceinline__ uint32_t spread8(uint32_t b8) {
-  uint32_t x = b8 & 0xFFu;
-  x = (x | (x << 12)) & 0x000F000Fu;
-  x = (x | (x << 6)) & 0x03030303u;
-  x = (x | (x << 3)) & 0x11111111u;
-  return x;
-}
-// Interleave the words of 4 vertices: bit 4r+i of y[q] = bit 8q+r of x[i],
-// so nibble r of y[q] holds source 8q+r for the 4 vertices.
-__device__ __forceinline__ void interleave4(const uint32_t (&x)[4], uint32_t (&y)[4]) {
-#pragma unroll
-  for (int q = 0; q < 4; q++)
-    y[q] = spread8(x[0] >> (8 * q)) | (spread8(x[1] >> (8 * q)) << 1) |
-           (spread8(x[2] >> (8 * q)) << 2) | (spread8(x[3] >> (8 * q)) << 3);
-}
-
 // In-register transpose of a 32 x 32 bit matrix, LSB-first: afterwards
 // bit r of A[j] is what bit j of A[r] was.  Five rounds of block swaps
 // (16, 8, 4, 2, 1), 16 masked delta swaps each; rows that are zero at

@@ -14,8 +14,8 @@
 #include "launch_common.cuh"
 
 // CTAs per SM the compiler must fit (register budget) for the two hottest
-// kernels; 0 leaves the budget to the compiler.  3 x 512 threads (at most
-// 42 registers) measured best on R-MAT scale 24: 48 warps per SM keep more
+// kernels; 0 leaves the budget to the compiler.  3 x 512 threads (40
+// registers) measured best on R-MAT scale 24: 48 warps per SM keep more
 // status gathers in flight than 2 x 512 at 64 registers, and 4 x 512 (32
 // registers) spills more than it gains.
 #ifndef IBFS_DL_BU_MINB

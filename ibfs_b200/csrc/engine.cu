@@ -460,14 +460,6 @@ void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int t
   p.sparse_div = o.sparse_push > 0 ? o.sparse_push : 0;
   p.col_vec = 1;
   p.vmap = g->vmap.as<int32_t>();
-  // Degrees are non-increasing in the internal order: the vertices above the
-  // thread-path limit form a prefix (rounded up to whole warps).  When each
-  // warp owns only a few 32-vertex ranges of the bottom-up sweep (small
-  // graphs), the warps that own the hub ranges would be the critical path,
-  // so the prefix then gets one warp per vertex; on large graphs the ranges
-  // average out and the per-lane sweep is faster (R-MAT scale 16: 1.26 ->
-  // 0.45 ms per run with the prefix pass; scale 24: 34.8 vs 40.7 ms without
-  // and with it).
   // Degrees are non-increasing in the internal order, so the edgeless
   // vertices form a suffix: the bottom-up sweeps stop before it (rounded up
   // to whole 32-vertex ranges).
@@ -483,6 +475,14 @@ void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int t
     // source reaches a vertex there (a directed graph's sinks can be reached)
     p.v_reach = g->col_max < p.v_nz ? p.v_nz : g->V;
   }
+  // The vertices above the thread-path limit form a prefix.  When each warp
+  // owns only a few 32-vertex ranges of the bottom-up sweep (small graphs), the
+  // warps that own the hub ranges would be the critical path, so the prefix is
+  // then spread over all warps: one vertex per warp in the own-kernel passes
+  // (R-MAT scale 16: 1.26 -> 0.45 ms per run), dealt out one per lane in the
+  // persistent kernel (same graph, 194 -> 174 us).  On large graphs the ranges
+  // average out and the plain sweep is faster (scale 24: 34.8 vs 40.7 ms
+  // without and with the prefix pass).
   const int64_t ranges_per_warp = ((g->V + 31) / 32) / std::max<int64_t>(1, (int64_t)g->sms * 64);
   if (ranges_per_warp < 8) {
     int64_t lo = 0, hi = g->V;
@@ -498,7 +498,7 @@ void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int t
 }
 
 // The output pointer and the store widths its alignment allows.
-void set_output_params(const ibfs_graph* g, int C, uint8_t* dout, Params* p) {
+void set_output_params(const ibfs_graph* g, uint8_t* dout, Params* p) {
   p->out = dout;
   p->vec_sm = (g->V % 16 == 0 && (reinterpret_cast<uintptr_t>(dout) & 15) == 0)  ? 16
               : (g->V % 4 == 0 && (reinterpret_cast<uintptr_t>(dout) & 3) == 0) ? 4
@@ -673,7 +673,10 @@ static ibfs_status order_on_host(ibfs_graph* g) {
 // launched.  ibfs_graph_from_csr on the host / on the GPU, best of 12: R-MAT
 // scale 10 (12 k edges) 0.97 / 0.82 ms, scale 11 (46 k) 1.62 / 1.21 ms, scale
 // 14 (0.43 M) 11.5 / 1.6 ms, scale 18 (7.6 M) 176 / 6.1 ms, scale 22 (128 M)
-// 1,987 / 110 ms.
+// 1,987 / 110 ms.  Short lists sort quickly: a path or grid of 16 to 65 k edges
+// takes 0.65 to 0.85 / 0.61 to 0.71 ms, but between there and 130 k edges, where
+// the scratch outgrows the allocator's small blocks, 0.9 to 1.3 / 1.3 to 1.4 ms
+// (grid of 261 k 1.6 / 1.45).
 static const int64_t kHostOrderEdges = 1 << 13;
 
 static ibfs_status upload_graph(ibfs_graph* g) {
@@ -1179,7 +1182,7 @@ static ibfs_status run_once(ibfs_graph* g, const int32_t* src, int64_t n, const 
   p.brec = reinterpret_cast<BatchRec*>(drun + rb.brec);
   p.lrec = g->d_lrec.as<LevelRec>();
   p.lrec_cap = kLrecCap;
-  set_output_params(g, rp.C, dout, &p);
+  set_output_params(g, dout, &p);
   // Per-batch done flags of the device loop, in mapped host memory, grown in
   // powers of two so that their address (baked into cached graphs) stays put.
   if (devloop && (size_t)rp.nbatches > g->done_cap) {

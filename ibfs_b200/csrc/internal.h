@@ -28,7 +28,6 @@ static inline uint64_t rnd(uint64_t seed, uint64_t stream, uint64_t i) {
   return mix64(mix64(seed ^ (stream * 0xD1B54A32D192ED03ull)) + i);
 }
 
-// Host CSR (int64 offsets, int32 column ids).
 // An array of the host CSR's size: not zeroed when it is sized (its pages are
 // first touched by whoever fills it, all cores at once), freed on destruction.
 // Throws std::bad_alloc like a vector.
@@ -67,6 +66,7 @@ class HostArray {
   size_t n_ = 0;
 };
 
+// Host CSR (int64 offsets, int32 column ids).
 struct HostCsr {
   int64_t V = 0, E = 0;
   HostArray<int64_t> beg;
@@ -130,7 +130,7 @@ const int32_t* graph_new_of_old(const ibfs_graph* g);  // caller id -> internal 
 // output pointer with the store widths its alignment allows.
 void fill_graph_params(const ibfs_graph* g, const ibfs_opts& o, int words, int threads,
                        Params* p);
-void set_output_params(const ibfs_graph* g, int C, uint8_t* dout, Params* p);
+void set_output_params(const ibfs_graph* g, uint8_t* dout, Params* p);
 }  // namespace ibfs
 
 namespace ibfs {

@@ -167,7 +167,7 @@ ibfs_status ServeLoop::init(ibfs_graph* g, const ibfs_opts& o, int G, int slots,
   p.cpg = graph_sms(g);
   p.db = db;
   p.layout = IBFS_LAYOUT_SOURCE_MAJOR;
-  set_output_params(g, C_, static_cast<uint8_t*>(arena), &p);
+  set_output_params(g, static_cast<uint8_t*>(arena), &p);
   p.groups = d_groups;
   p.brec = reinterpret_cast<BatchRec*>(db_base + o_brec);
   p.lrec = nullptr;

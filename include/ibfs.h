@@ -108,8 +108,8 @@ typedef struct ibfs_opts {
                               barrier, so every wait runs out (IBFS_ERR_TIMEOUT)  */
     int32_t occupancy;     /* persistent kernel register budget / warps per SM:
                               0: 512 threads x 2 CTAs (64 regs; x 1, 128 regs, when
-                              the grid has at most one CTA per SM), 1: 256 x 6 (42),
-                              2: 256 x 8 (32), 3: 512 x 1 (128)                 */
+                              the grid has at most one CTA per SM), 1: 256 x 6 (40),
+                              2: 256 x 7 (32), 3: 512 x 1 (128)                 */
     int32_t bu_filter;     /* bottom-up reads a neighbour's status only when the
                               previous frontier bitmap has it (exact: no other
                               neighbour can add a bit): 1 on every level, 0 off,
