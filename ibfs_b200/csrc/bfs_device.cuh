@@ -1442,18 +1442,16 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   const uint32_t* front = chg_at(gb, p, level - 1);
   uint32_t* out = chg_at(gb, p, level);
   const int lane = t.lane;
-  // FUSED counters (as inspect_phase).  A degree is below 2^31 here; a sum of
-  // one thread's degrees passes 2^32 only in a graph of that many edges, and
-  // then hands the carry to the level's -- in the persistent kernel, whose team
-  // may be one CTA.  The own-kernel pass has the whole GPU's threads, so one of
-  // them would have to own lists of 2^32 edges; these two sums only steer the
-  // direction choice, and the carry costs its sweep 1.5 % (grid 4096^2).
+  // FUSED counters (as inspect_phase).  32 bits hold a thread's degree sums: a
+  // degree is below 2^31 here, and in the degree order each later vertex of a
+  // thread has at most the average degree of the round of vertices before it, so
+  // that they add up to at most E / threads (E / warps in the own-kernel prefix
+  // loop), below 2^31 for every E that fits the GPU.  (A caller's own order, ibfs_run_static_scratch, could pass that
+  // only with lists full of duplicates; the sums steer the direction choice and
+  // no depth.)  The kernels are sensitive here: handing a carry on instead cost
+  // the grid 1.5 % in the device loop and 4 % in the persistent kernel.
   uint32_t f_mf = 0, f_cnt = 0, f_cdeg = 0;
   unsigned long long f_teps = 0;
-  auto add_degree = [](uint32_t* sum, uint32_t deg, unsigned long long* total) {
-    *sum += deg;
-    if (!RO && *sum < deg) atomicAdd(total, 1ull << 32);
-  };
   const bool first_plane = (level & (level - 1)) == 0;
   const int pb = __ffs(level) - 1;
   bool range = false;
@@ -1510,9 +1508,9 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
         if (epi) {
           const uint32_t deg = (uint32_t)deg_v;
           f_cnt += 1;
-          add_degree(&f_mf, deg, &par->mf);
+          f_mf += deg;
           f_teps += (unsigned long long)deg * pop;
-          if (comp) add_degree(&f_cdeg, deg, &par->cdeg);
+          if (comp) f_cdeg += deg;
           if (!depth_ok) range = true;
           atomicOr(out + (v >> 5), 1u << (v & 31));
         }
@@ -1696,9 +1694,9 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
       if (epi) {
         const uint32_t deg = (uint32_t)deg_v;
         f_cnt += 1;
-        add_degree(&f_mf, deg, &par->mf);
+        f_mf += deg;
         f_teps += (unsigned long long)deg * pop;
-        if (comp) add_degree(&f_cdeg, deg, &par->cdeg);
+        if (comp) f_cdeg += deg;
         if (!depth_ok) range = true;
       }
       uint32_t* q0 = gb.planes + (size_t)v * WORDS;
