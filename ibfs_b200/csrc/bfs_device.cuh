@@ -1446,10 +1446,11 @@ __device__ void bu_phase(const Params& p, const GroupBufs& gb, int level,
   // degree is below 2^31 here, and in the degree order each later vertex of a
   // thread has at most the average degree of the round of vertices before it, so
   // that they add up to at most E / threads (E / warps in the own-kernel prefix
-  // loop), below 2^31 for every E that fits the GPU.  (A caller's own order, ibfs_run_static_scratch, could pass that
-  // only with lists full of duplicates; the sums steer the direction choice and
-  // no depth.)  The kernels are sensitive here: handing a carry on instead cost
-  // the grid 1.5 % in the device loop and 4 % in the persistent kernel.
+  // loop), below 2^31 for every E that fits the GPU.  (A caller's own order,
+  // ibfs_run_static_scratch, could pass that only with lists full of
+  // duplicates; the sums steer the direction choice and no depth.)  The kernels
+  // are sensitive here: handing a carry on instead cost the grid 1.5 % in the
+  // device loop and deep grids 4 % in the persistent kernel.
   uint32_t f_mf = 0, f_cnt = 0, f_cdeg = 0;
   unsigned long long f_teps = 0;
   const bool first_plane = (level & (level - 1)) == 0;
